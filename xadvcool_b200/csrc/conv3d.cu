@@ -12,9 +12,15 @@
 //             fixed order.
 //
 // Ci and Co must be multiples of 16 (the model pads its 3 input channels and 5 output channels to 16).
+#include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <array>
+#include <atomic>
+#include <cmath>
 #include <cstdint>
+#include <map>
+#include <mutex>
 
 #include "xac_internal.cuh"
 
@@ -54,21 +60,7 @@ __device__ __forceinline__ long long neighbour(const VoxelCoord& c, int dz, int 
   return (((long long)c.n * s.D + z) * s.H + y) * s.W + x;
 }
 
-// ---- forward / data grad on the 5th-generation tensor cores (tcgen05) ------------------------------------
-// One CTA of 128 threads computes a 128-voxel x Co tile: D[128][Co] (FP32, in tensor memory) =
-// sum over K = taps x Ci of A[voxel][k] * B[co][k]. K is walked in stages of one tap x BK channels:
-//   * all 128 threads gather the stage's operands into shared memory with 16-byte cp.async copies (zero-filled
-//     where the neighbour is outside the volume), A row r = voxel m0 + r, B row n = output channel n;
-//   * one thread issues the stage's BK/16 tcgen05.mma (kind::f16, BF16 in, FP32 accumulate) and a
-//     tcgen05.commit that frees the stage when those MMAs have read it;
-//   * a ring of kStages stages overlaps the gathers with the MMAs (mbarriers "full" and "empty").
-// Shared-memory operand layout (K-major, no swizzle): 16-byte chunks of 8 channels, [BK/8][rows][8], so a core
-// matrix (8 rows x 16 bytes) is 128 contiguous bytes, 8-row groups are 128 bytes apart (stride byte offset) and
-// the two 8-channel halves of one K = 16 MMA step are rows*16 bytes apart (leading byte offset).
-// Epilogue: warp w reads tensor-memory lanes 32w..32w+31 (its voxels) 16 columns at a time, adds the bias,
-// applies GELU if asked, and stores BF16 or FP32.
-// Every wait is bounded: a wait that runs out sets g_conv_status, the CTA stops issuing work, waits (bounded) for
-// the MMAs it issued, frees its tensor memory and returns.
+// ---- shared pieces of the tcgen05 kernels ----------------------------------------------------------------
 constexpr int kTcM = 128;
 constexpr int kTcStages = 4;
 constexpr uint32_t kTcSpin = 1u << 22;
@@ -95,6 +87,41 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   atomicOr(&g_conv_status, 1u);
   return false;
 }
+// bounded wait that also ends when another role of the CTA gave up; one that runs out raises the CTA's abort flag
+__device__ __forceinline__ bool mbar_wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_v) {
+  for (uint32_t i = 0; i < kTcSpin; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if (*abort_v) return false;
+  }
+  atomicOr(&g_conv_status, 1u);
+  *abort_v = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// tiled TMA loads: the innermost coordinate is a multiple of 16 channels (32 bytes); boxes may start or end outside
+// the tensor, where they read zeros
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
+                                            uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
+      "[%7];"
+      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+      : "memory");
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -107,7 +134,8 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// shared-memory matrix descriptor: K-major, no swizzle (layout type 0), descriptor version 1
+// shared-memory matrix descriptor: no swizzle (layout type 0 in bits 61..63), descriptor version 1
+constexpr uint32_t kSwizzle128 = 2, kSwizzle64 = 4, kSwizzle32 = 6;
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
@@ -116,11 +144,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 __host__ __device__ constexpr uint32_t tc_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
 }
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+// a, b: descriptors as low and high words
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                       uint32_t idesc, uint32_t accum) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(tmem_d), "l"(a), "l"(b), "r"(idesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\t"
+      "mov.b64 b, {%3, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
+      ::"r"(tmem_d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accum));
+}
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+  tc_mma(tmem_d, (uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32), idesc, accum);
+}
+// one lane of a converged warp, the same one each time; the compiler then knows that the code under it runs in a
+// single thread and keeps the MMA operands in uniform registers without a loop around every instruction
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -137,150 +177,396 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-struct TcConv {
-  int BK;          // channels per stage (16..64, divides Ci)
-  int kt;          // stages of K: taps * Ci / BK
-  uint32_t ncols;  // tensor-memory columns allocated (power of two >= max(32, Co))
+// ---- forward / data grad on the 5th-generation tensor cores (tcgen05) ------------------------------------
+// Bound: for Co <= 64 the tensor core's reads of the activation operand from shared memory (4 KB per 128 voxels x 16
+// channels: 39 cycles an MMA for Co = 16, 48 for 64, where the products alone would take 8 and 32). The kernel
+// before this one copied that operand from L2 once per tap, one 16-byte copy per thread, and one thread issued its
+// MMAs from a loop. Here a plane of input voxels with its halo is copied once and the 27 taps read it in place:
+//
+//   * A unit of work is a tile of bx x by voxels of one z plane (x Co, or a slice of nb channels of it). Its input is
+//     three z planes of by + 2 rows of P = bx + 2 voxels; TMA boxes fill the part outside the volume with zeros.
+//   * A plane lies in shared memory as Ci / KB blocks of [R voxels][KB channels] (K-major, swizzle of the row size:
+//     KB = 64, 32, 16 channels are 128, 64, 32 bytes), so the A operand of tap (dz,dy,dx) is the plane's rows
+//     m + dy*P + dx, m = y*P + x: the same bytes from another start address.
+//   * The accumulator rows m run over the flattened tile, mt blocks of 128 rows; rows with x >= bx are halo columns
+//     and are dropped by the epilogue (2 of P).
+//   * A CTA walks a contiguous range of units, z fastest. When its planes are kept (march) a plane is copied once
+//     for the three units that read it, into a ring of NS planes; the tap order has dz outermost, so the oldest
+//     plane is free after the first third of a unit and the next one is on its way during the rest.
+//   * Weights: all of them resident where they fit beside the planes, otherwise a ring of stages of one tap (all of its
+//     channels where Ci / KB is at most 3, else KB of them).
+//
+// The products of an output are added in the order tap, then channel, whatever the tile.
+//
+// Measured on a B200, the kernel before -> this one (same bits): 16 -> 16 channels at 32x128x152 217 -> 35 us, at batch 4
+// 808 -> 113 (the MMAs alone 77), 48 -> 16 2203 -> 270, 96 -> 32 at 16x64x76 755 -> 131, 192 -> 64 at 8x32x38 357 -> 74.
+//
+// Roles: warps 0-15 epilogue, 16-19 issue the MMAs (warp 16 + k those of the accumulator blocks k, k + 4, ...), 20
+// copies input planes and 21 weights. Accumulators are double-buffered in tensor memory where they fit, so the epilogue
+// of a unit runs under the MMAs of the next.
+// Every wait is bounded: a wait that runs out sets g_conv_status and the CTA's abort flag, every role leaves its
+// loop, and the CTA waits (bounded) for its copies and MMAs in flight, frees its tensor memory and returns.
+constexpr int kFwdThreads = 704;
+constexpr int kEpiWarps = 16;
+constexpr int kMmaWarps = 4;
+constexpr int kMaxPlanes = 4;
+constexpr int kMaxBStages = 8;
+
+struct FwdPlan {
+  int bx, by, P, nxt, nyt;  // tile, row length with halo, tiles along x and y
+  int mt, R;                // blocks of 128 accumulator rows; voxels of a stored plane
+  int NS, march;            // planes in the ring; 1: planes are kept from one z to the next
+  int nb, nsplit;           // output channels of a unit, slices of Co
+  int KB, G;                // channels of a block, blocks of a weight stage
+  int bs, resident;         // weight stages held, 1: all weights held
+  int nbuf;                 // accumulator buffers
+  uint32_t ncols;           // tensor-memory columns allocated
+  long long units;
+  int ctas;
+  size_t smem;
 };
 
-__global__ void __launch_bounds__(128, 1) conv_fwd_tc_kernel(const __nv_bfloat16* __restrict__ in,
-                                                             const __nv_bfloat16* __restrict__ w,
-                                                             const float* __restrict__ bias, ConvShape s, int act,
-                                                             TcConv t, __nv_bfloat16* __restrict__ out_bf16,
-                                                             float* __restrict__ out_f32) {
+// barriers, by number
+struct FwdBars {
+  uint32_t b0;
+  __device__ __forceinline__ uint32_t afull(int i) const { return b0 + 8u * i; }
+  __device__ __forceinline__ uint32_t aempty(int i) const { return b0 + 8u * (kMaxPlanes + i); }
+  __device__ __forceinline__ uint32_t bfull(int i) const { return b0 + 8u * (2 * kMaxPlanes + i); }
+  __device__ __forceinline__ uint32_t bempty(int i) const { return b0 + 8u * (2 * kMaxPlanes + kMaxBStages + i); }
+  __device__ __forceinline__ uint32_t cfull(int i) const { return b0 + 8u * (2 * kMaxPlanes + 2 * kMaxBStages + i); }
+  __device__ __forceinline__ uint32_t cempty(int i) const {
+    return b0 + 8u * (2 * kMaxPlanes + 2 * kMaxBStages + 2 + i);
+  }
+  __device__ __forceinline__ uint32_t done() const { return b0 + 8u * (2 * kMaxPlanes + 2 * kMaxBStages + 4); }
+  static constexpr int kCount = 2 * kMaxPlanes + 2 * kMaxBStages + 5;
+};
+
+struct MmaRole {
+  uint32_t tmem;
+  uint32_t a, b, hi;           // descriptors of the first plane and weight stage (low words), their high word
+  uint32_t plane16, bblk16;    // sizes of a plane and of a weight block in 16-byte units
+  FwdBars bar;
+  int nd, nst, taps;           // stages of a tap
+  volatile int* abort_v;
+};
+
+// KC steps of 16 channels (32 bytes apart) for NT accumulator blocks; a, b: low words of the descriptors
+template <int KC, int NT>
+__device__ __forceinline__ void issue_stage(uint32_t d, uint32_t dstep, uint32_t a, uint32_t b, uint32_t hi,
+                                            uint32_t idesc, uint32_t accum) {
+  constexpr uint32_t kBlock = kMmaWarps * kTcM * KC * 2;  // four blocks of 128 rows of KC * 32 bytes, in 16 bytes
+#pragma unroll
+  for (int c = 0; c < KC; ++c)
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+      tc_mma(d + (uint32_t)t * dstep, a + (uint32_t)(2 * c) + (uint32_t)t * kBlock, hi, b + (uint32_t)(2 * c), hi, idesc,
+             c == 0 ? accum : 1u);
+}
+
+// one weight stage: G blocks of KC steps; ablk, bblk: distances of the blocks
+template <int KC, int G, int NT>
+__device__ __forceinline__ void issue_tap(uint32_t d, uint32_t dstep, uint32_t a, uint32_t ablk, uint32_t b,
+                                          uint32_t bblk, uint32_t hi, uint32_t idesc, uint32_t accum) {
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+    issue_stage<KC, NT>(d, dstep, a + (uint32_t)g * ablk, b + (uint32_t)g * bblk, hi, idesc, g == 0 ? accum : 1u);
+}
+
+// The MMAs of one warp over the CTA's units (the whole warp waits, one lane issues). An MMA in a loop of its own
+// costs its thread 180-250 cycles, in straight-line code 45-120, so the taps of a plane (or of a row of it) are
+// unrolled where the weights are resident, and four warps issue side by side.
+template <int KC, int G, int NT>
+__device__ __forceinline__ void mma_role(const MmaRole& m, const ConvShape& s, const FwdPlan& pl, int t0, int issuer,
+                                         long long u_begin, long long u_end) {
+  constexpr uint32_t kRow = KC * 2;  // a voxel's row in 16-byte units
+  const int nb = pl.nb, P = pl.P, D = s.D, nd = m.nd, nst = m.nst;
+  const uint32_t idesc = tc_idesc(nb);
+  const uint32_t abase = m.a + (uint32_t)(t0 * kTcM) * kRow, ablk = (uint32_t)pl.R * kRow;
+  const uint32_t bblk = pl.resident ? (uint32_t)m.taps * m.bblk16 : m.bblk16;
+  const uint32_t dstep = (uint32_t)(kMmaWarps * nb);
+  int seq0 = 0, cnt = 0, st = 0;
+  uint32_t bpar = 0;
+  if (pl.resident) {
+    if (!mbar_wait_or_abort(m.bar.bfull(0), 0, m.abort_v)) return;
+    tc_fence_after();
+  }
+  for (long long u = u_begin; u < u_end;) {
+    const int z0 = (int)(u % D);
+    const int nz = (int)((u_end - u < D - z0) ? u_end - u : D - z0);
+    for (int i = 0; i < nz; ++i, ++cnt) {
+      const int buf = cnt % pl.nbuf;
+      if (cnt >= pl.nbuf && !mbar_wait_or_abort(m.bar.cempty(buf), ((cnt / pl.nbuf) - 1) & 1, m.abort_v)) return;
+      tc_fence_after();
+      const uint32_t acc = m.tmem + (uint32_t)((buf * pl.mt + t0) * nb);
+      for (int dz = 0; dz < nd; ++dz) {
+        const int sq = seq0 + (pl.march ? i + dz : i * nd + dz), slot = sq % pl.NS;
+        if (!mbar_wait_or_abort(m.bar.afull(slot), (sq / pl.NS) & 1, m.abort_v)) return;
+        tc_fence_after();
+        const uint32_t arow = abase + (uint32_t)slot * m.plane16;
+        if (pl.resident && nst == 1 && nd == 3) {
+          if (issuer) {
+            constexpr int kRows = KC * G * NT <= 4 ? 3 : 1;  // rows of taps in one straight run
+#pragma unroll 1
+            for (int dy0 = 0; dy0 < 3; dy0 += kRows) {
+#pragma unroll
+              for (int k = 0; k < 3 * kRows; ++k) {
+                const int dy = dy0 + k / 3, dx = k % 3;
+                issue_tap<KC, G, NT>(acc, dstep, arow + (uint32_t)(dy * P + dx) * kRow, ablk,
+                                     m.b + (uint32_t)(dz * 9 + dy * 3 + dx) * m.bblk16, bblk, m.hi, idesc,
+                                     (dz > 0 || dy > 0 || dx > 0) ? 1u : 0u);
+              }
+            }
+          }
+        } else {
+          for (int dyx = 0; dyx < nd * nd; ++dyx) {
+            const uint32_t a = arow + (uint32_t)(dyx / nd * P + dyx % nd) * kRow;
+            for (int k = 0; k < nst; ++k) {
+              if (!pl.resident) {
+                if (!mbar_wait_or_abort(m.bar.bfull(st), bpar, m.abort_v)) return;
+                tc_fence_after();
+              }
+              if (issuer) {
+                const int blk = pl.resident ? k * G * m.taps + dz * nd * nd + dyx : st * G;
+                issue_tap<KC, G, NT>(acc, dstep, a + (uint32_t)(k * G) * ablk, ablk,
+                                     m.b + (uint32_t)blk * m.bblk16, bblk, m.hi, idesc,
+                                     (dz > 0 || dyx > 0 || k > 0) ? 1u : 0u);
+                if (!pl.resident) tc_commit(m.bar.bempty(st));
+              }
+              if (++st == pl.bs) {
+                st = 0;
+                bpar ^= 1u;
+              }
+            }
+          }
+        }
+        if (issuer && (!pl.march || dz == 0 || i == nz - 1)) tc_commit(m.bar.aempty(slot));
+        __syncwarp();
+      }
+      if (issuer) tc_commit(m.bar.cfull(buf));
+      __syncwarp();
+    }
+    seq0 += pl.march ? nz + nd - 1 : nz * nd;
+    u += nz;
+  }
+}
+
+// strip = (slice of Co, batch item, y tile, x tile)
+struct Strip {
+  int n0, n, y0, x0;
+};
+__device__ __forceinline__ Strip strip_of(long long strip, const FwdPlan& pl, const ConvShape& s) {
+  Strip t;
+  unsigned v = (unsigned)strip;
+  t.x0 = (int)(v % pl.nxt) * pl.bx;
+  v /= pl.nxt;
+  t.y0 = (int)(v % pl.nyt) * pl.by;
+  v /= pl.nyt;
+  t.n = (int)(v % s.N);
+  t.n0 = (int)(v / s.N) * pl.nb;
+  return t;
+}
+
+__global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_constant__ CUtensorMap tin,
+                                                                  const __grid_constant__ CUtensorMap tw,
+                                                                  const float* __restrict__ bias, ConvShape s, int act,
+                                                                  FwdPlan pl, __nv_bfloat16* __restrict__ out_bf16,
+                                                                  float* __restrict__ out_f32) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[2 * kTcStages + 1];  // full[s], empty[s], done
+  __shared__ __align__(8) uint64_t bars[FwdBars::kCount];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int Co = s.Co, BK = t.BK, chunks = BK >> 3;
-  const long long V = (long long)s.N * s.D * s.H * s.W;
-  const long long m0 = (long long)blockIdx.x * kTcM;
-  const uint32_t a_bytes = kTcM * BK * 2, b_bytes = (uint32_t)Co * BK * 2, stage_bytes = a_bytes + b_bytes;
-  const uint32_t sbase = smem_addr(smem);
-  const uint32_t bar0 = smem_addr(bars);
-  auto full = [&](int st) { return bar0 + 8u * st; };
-  auto empty = [&](int st) { return bar0 + 8u * (kTcStages + st); };
-  const uint32_t done_bar = bar0 + 8u * (2 * kTcStages);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int Co = s.Co, kr = s.ksize >> 1, nd = s.ksize, taps = nd * nd * nd, nb = pl.nb, P = pl.P, D = s.D;
+  const int nkc = s.Ci / pl.KB;
+  const int nmw = pl.mt < kMmaWarps ? pl.mt : kMmaWarps;  // warps that issue MMAs
+  const uint32_t row_bytes = (uint32_t)pl.KB * 2u;
+  const uint32_t plane_bytes = (uint32_t)nkc * pl.R * row_bytes, bblk_bytes = (uint32_t)nb * row_bytes;
+  const uint32_t bstage_bytes = (uint32_t)pl.G * bblk_bytes;
+  const uint32_t a0 = smem_addr(smem), b0 = a0 + pl.NS * plane_bytes;
+  const FwdBars bar{smem_addr(bars)};
 
   if (tid == 0) {
-    for (int st = 0; st < kTcStages; ++st) {
-      mbar_init(full(st), 128);
-      mbar_init(empty(st), 1);
+    for (int i = 0; i < kMaxPlanes; ++i) {
+      mbar_init(bar.afull(i), 1);
+      mbar_init(bar.aempty(i), nmw);
     }
-    mbar_init(done_bar, 1);
+    for (int i = 0; i < kMaxBStages; ++i) {
+      mbar_init(bar.bfull(i), 1);
+      mbar_init(bar.bempty(i), nmw);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar.cfull(i), nmw);
+      mbar_init(bar.cempty(i), 32 * kEpiWarps);
+    }
+    mbar_init(bar.done(), nmw);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
-                 "r"(t.ncols));
+                 "r"(pl.ncols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
+  volatile int* abort_v = &abort_flag;
+  const long long u_begin = pl.units * blockIdx.x / gridDim.x, u_end = pl.units * (blockIdx.x + 1) / gridDim.x;
 
-  // this thread's A row: voxel m0 + tid
-  const long long v = m0 + tid;
-  const bool vrow = v < V;
-  const VoxelCoord vc = decode(vrow ? v : 0, s);
-  const int ci_chunks = s.Ci / BK;
-  const uint32_t idesc = tc_idesc(Co);
-
-  auto load_stage = [&](int k, int st) {
-    const int tap = k / ci_chunks, kc = k - tap * ci_chunks;
-    const int dz = s.ksize == 3 ? tap / 9 - 1 : 0, dy = s.ksize == 3 ? (tap / 3) % 3 - 1 : 0,
-              dx = s.ksize == 3 ? tap % 3 - 1 : 0;
-    const long long nb = vrow ? neighbour(vc, dz, dy, dx, s) : -1;
-    const uint32_t a_st = sbase + (uint32_t)st * stage_bytes, b_st = a_st + a_bytes;
-    const __nv_bfloat16* asrc = nb >= 0 ? in + nb * s.Ci + kc * BK : in;
-    for (int j = 0; j < chunks; ++j)
-      cp_async16(a_st + (uint32_t)(j * kTcM + tid) * 16u, asrc + (nb >= 0 ? j * 8 : 0), nb >= 0 ? 16u : 0u);
-    const __nv_bfloat16* wt = w + ((long long)tap * Co) * s.Ci + kc * BK;
-    for (int e = tid; e < Co * chunks; e += 128) {
-      const int n = e / chunks, j = e - n * chunks;
-      cp_async16(b_st + (uint32_t)(j * Co + n) * 16u, wt + (long long)n * s.Ci + j * 8, 16u);
-    }
-  };
-  auto mma_stage = [&](int k, int st) {
-    const uint32_t a_st = sbase + (uint32_t)st * stage_bytes, b_st = a_st + a_bytes;
-    for (int q = 0; q < BK / 16; ++q) {
-      const uint64_t ad = smem_desc(a_st + (uint32_t)(2 * q) * kTcM * 16u, kTcM * 16u, 128u);
-      const uint64_t bd = smem_desc(b_st + (uint32_t)(2 * q) * Co * 16u, (uint32_t)Co * 16u, 128u);
-      tc_mma(tmem, ad, bd, idesc, (k > 0 || q > 0) ? 1u : 0u);
-    }
-    tc_commit(empty(st));
-  };
-
-  const int KT = t.kt;
-  for (int k = 0; k < KT + kTcStages - 1; ++k) {
-    if (k < KT) {
-      const int st = k % kTcStages;
-      if (k >= kTcStages && !mbar_wait(empty(st), ((k / kTcStages) - 1) & 1)) abort_flag = 1;
-      if (abort_flag) break;
-      load_stage(k, st);
-    }
-    cp_async_commit();
-    const int kc = k - (kTcStages - 1);  // the stage whose copies this thread now completes
-    if (kc >= 0) {
-      cp_async_wait<kTcStages - 1>();
-      fence_proxy_async();
-      mbar_arrive(full(kc % kTcStages));
-      if (warp == 0) {  // the whole warp waits, lane 0 issues
-        if (mbar_wait(full(kc % kTcStages), (kc / kTcStages) & 1)) {
-          tc_fence_after();
-          if (lane == 0) mma_stage(kc, kc % kTcStages);
-        } else {
-          abort_flag = 1;
+  if (warp == kEpiWarps + kMmaWarps) {
+    // ---- input planes: one thread starts the boxes of a plane, one per block of KB channels
+    if (lane == 0) {
+      const uint32_t bytes = (uint32_t)nkc * (uint32_t)(P * (pl.by + 2 * kr)) * row_bytes;
+      int slot = 0, seq = 0;
+      uint32_t par = 1;  // parity of the wait for room: passes at once in the first round
+      auto load_plane = [&](const Strip& t, int z) -> bool {
+        if (!mbar_wait_or_abort(bar.aempty(slot), par, abort_v)) return false;
+        mbar_expect_tx(bar.afull(slot), bytes);
+        for (int k = 0; k < nkc; ++k)
+          tma_load_5d(a0 + (uint32_t)slot * plane_bytes + (uint32_t)(k * pl.R) * row_bytes, &tin, k * pl.KB, t.x0 - kr,
+                      t.y0 - kr, z, t.n, bar.afull(slot));
+        ++seq;
+        if (++slot == pl.NS) {
+          slot = 0;
+          par ^= 1u;
         }
-        __syncwarp();
+        return true;
+      };
+      bool ok = true;
+      for (long long u = u_begin; ok && u < u_end;) {
+        const long long strip = u / D;
+        const int z0 = (int)(u - strip * D);
+        const int nz = (int)((u_end - u < D - z0) ? u_end - u : D - z0);
+        const Strip t = strip_of(strip, pl, s);
+        if (pl.march) {
+          for (int i = 0; ok && i < nz + 2 * kr; ++i) ok = load_plane(t, z0 - kr + i);
+        } else {
+          for (int z = z0; ok && z < z0 + nz; ++z)
+            for (int d = 0; ok && d < nd; ++d) ok = load_plane(t, z - kr + d);
+        }
+        u += nz;
+      }
+      // an abort may leave copies that no role waited for: let them land before the block's memory goes back
+      if (*abort_v)
+        for (int k = seq > pl.NS ? seq - pl.NS : 0; k < seq; ++k) mbar_wait(bar.afull(k % pl.NS), (k / pl.NS) & 1);
+    }
+  } else if (warp == kEpiWarps + kMmaWarps + 1) {
+    // ---- weights: all of them at once, or the stages of one unit again and again (with the unit's slice of Co)
+    if (lane == 0) {
+      if (pl.resident) {
+        mbar_expect_tx(bar.bfull(0), (uint32_t)(taps * nkc) * bblk_bytes);
+        for (int k = 0; k < nkc; ++k)
+          tma_load_3d(b0 + (uint32_t)(k * taps) * bblk_bytes, &tw, k * pl.KB, 0, 0, bar.bfull(0));
+        if (*abort_v) mbar_wait(bar.bfull(0), 0);
+      } else {
+        int st = 0;
+        long long seq = 0;
+        uint32_t par = 1;
+        bool ok = true;
+        for (long long u = u_begin; ok && u < u_end; ++u) {
+          const Strip t = strip_of(u / D, pl, s);
+          for (int tap = 0; ok && tap < taps; ++tap)
+            for (int k = 0; k < nkc; k += pl.G) {
+              if (!mbar_wait_or_abort(bar.bempty(st), par, abort_v)) {
+                ok = false;
+                break;
+              }
+              mbar_expect_tx(bar.bfull(st), bstage_bytes);
+              for (int g = 0; g < pl.G; ++g)
+                tma_load_3d(b0 + (uint32_t)st * bstage_bytes + (uint32_t)g * bblk_bytes, &tw, (k + g) * pl.KB, t.n0, tap,
+                            bar.bfull(st));
+              ++seq;
+              if (++st == pl.bs) {
+                st = 0;
+                par ^= 1u;
+              }
+            }
+        }
+        if (*abort_v)
+          for (long long k = seq > pl.bs ? seq - pl.bs : 0; k < seq; ++k)
+            mbar_wait(bar.bfull((int)(k % pl.bs)), (uint32_t)(k / pl.bs) & 1u);
       }
     }
-    if (abort_flag) break;
+  } else if (warp >= kEpiWarps) {
+    // ---- MMA issue: accumulator blocks t0, t0 + 4, ...
+    const int t0 = warp - kEpiWarps;
+    if (t0 < nmw) {
+      const uint64_t desc = smem_desc(0, 16u, 8u * row_bytes) |
+                            ((uint64_t)(pl.KB == 64 ? kSwizzle128 : (pl.KB == 32 ? kSwizzle64 : kSwizzle32)) << 61);
+      const uint32_t dlo = (uint32_t)desc, dhi = (uint32_t)(desc >> 32);
+      const MmaRole m{tmem, dlo + (a0 >> 4), dlo + (b0 >> 4), dhi, plane_bytes >> 4, bblk_bytes >> 4, bar, nd,
+                      nkc / pl.G, taps, abort_v};
+      const int nt = (pl.mt - t0 + kMmaWarps - 1) / kMmaWarps, kc = pl.KB >> 4;
+      const int issuer = elect_one() ? 1 : 0;
+#define XAC_ROLE(KC, GG)                                                    \
+  if (kc == KC && pl.G == GG) {                                             \
+    if (nt == 1) mma_role<KC, GG, 1>(m, s, pl, t0, issuer, u_begin, u_end); \
+    else mma_role<KC, GG, 2>(m, s, pl, t0, issuer, u_begin, u_end);         \
   }
-  cp_async_wait<0>();
-  // the last commit (or, after an abort, a fresh one) arrives on done_bar when every issued MMA has finished
-  if (tid == 0) tc_commit(done_bar);
-  const int drained = mbar_wait(done_bar, 0) ? 1 : 0;
-  const bool ok = __syncthreads_and(drained) && !abort_flag;  // uniform: every thread has left the loop
-  tc_fence_after();
-  if (ok) {
-    const long long vr = m0 + warp * 32 + lane;
-    for (int c0 = 0; c0 < Co; c0 += 16) {
-      float x[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, x);
-      if (vr < V) {
+      XAC_ROLE(1, 1) XAC_ROLE(2, 1) XAC_ROLE(4, 1) XAC_ROLE(1, 3) XAC_ROLE(2, 3) XAC_ROLE(4, 2) XAC_ROLE(4, 3)
+#undef XAC_ROLE
+      // arrives when every MMA issued has finished
+      if (issuer) tc_commit(bar.done());
+    }
+  } else {
+    // ---- epilogue: warp w reads tensor-memory lanes 32 (w % 4)..; blocks x 16-column groups go round the warps
+    int cnt = 0;
+    const int quad = warp & 3;
+    for (long long u = u_begin; u < u_end; ++u, ++cnt) {
+      const int buf = cnt % pl.nbuf;
+      if (!mbar_wait_or_abort(bar.cfull(buf), (cnt / pl.nbuf) & 1, abort_v)) break;
+      tc_fence_after();
+      const long long strip = u / D;
+      const int z = (int)(u - strip * D);
+      const Strip t = strip_of(strip, pl, s);
+      const int groups = nb >> 4;
+      for (int it = warp >> 2; it < pl.mt * groups; it += kEpiWarps / 4) {
+        const int b = it / groups, c0 = (it - b * groups) << 4;
+        const int m = b * kTcM + quad * 32 + lane;
+        const int y = m / P, x = m - y * P;
+        const int gy = t.y0 + y, gx = t.x0 + x;
+        const bool valid = x < pl.bx && y < pl.by && gy < s.H && gx < s.W;
+        const long long o = ((((long long)t.n * D + z) * s.H + gy) * s.W + gx) * Co + t.n0;
+        {
+          float v[16];
+          __syncwarp();
+          tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)((buf * pl.mt + b) * nb + c0), v);
+          if (!valid) continue;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float y = x[i] + (bias ? __ldg(bias + c0 + i) : 0.0f);
-          x[i] = act == 1 ? gelu(y) : y;
-        }
-        if (out_bf16) {
-          uint4 pk[2];
-          uint32_t* pw = reinterpret_cast<uint32_t*>(pk);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            __nv_bfloat162 b2 = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-            pw[i] = *reinterpret_cast<uint32_t*>(&b2);
+          for (int i = 0; i < 16; ++i) {
+            const float yv = v[i] + (bias ? __ldg(bias + t.n0 + c0 + i) : 0.0f);
+            v[i] = act == 1 ? gelu(yv) : yv;
           }
-          uint4* dst = reinterpret_cast<uint4*>(out_bf16 + vr * Co + c0);
-          dst[0] = pk[0];
-          dst[1] = pk[1];
-        } else {
-          float4* dst = reinterpret_cast<float4*>(out_f32 + vr * Co + c0);
+          if (out_bf16) {
+            uint4 pk[2];
+            uint32_t* pw = reinterpret_cast<uint32_t*>(pk);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) dst[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+            for (int i = 0; i < 8; ++i) {
+              __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+              pw[i] = *reinterpret_cast<uint32_t*>(&b2);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(out_bf16 + o + c0);
+            dst[0] = pk[0];
+            dst[1] = pk[1];
+          } else {
+            float4* dst = reinterpret_cast<float4*>(out_f32 + o + c0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          }
         }
       }
+      tc_fence_before();
+      mbar_arrive(bar.cempty(buf));
     }
   }
-  tc_fence_before();
+  // every MMA issued has finished before the tensor memory goes back
+  __syncwarp();
+  mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(t.ncols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(pl.ncols));
   }
 }
 
@@ -471,6 +757,172 @@ int check_shape(const ConvShape& s) {
   return XAC_OK;
 }
 
+
+// ---- host: the forward tile ---------------------------------------------------------------------------------
+// The tile is a pure function of the shape: the cheapest of all tiles that fit, by a model of one CTA's time (the
+// longest CTA decides): MMAs at the measured rate (39 cycles for 128 voxels x 16 channels x Co = 16, 48 for 64, 64 for 128)
+// against the bytes copied from L2 at about 22 B/clk per SM, plus a fixed cost per unit and per CTA. It picks the
+// slice of Co, the tile, the plane ring and resident or streamed weights.
+constexpr size_t kSmemLimit = 231000;  // dynamic shared memory of a CTA (227 KB less the static part)
+
+int sm_count(int* out) {
+  int dev = 0;
+  XAC_CUDA(cudaGetDevice(&dev));
+  XAC_CUDA(cudaDeviceGetAttribute(out, cudaDevAttrMultiProcessorCount, dev));
+  return XAC_OK;
+}
+
+// Raises a kernel's dynamic shared-memory limit once per device (the attribute belongs to the device's context).
+enum { kFwdSlot = 0, kWgSlot = 1, kSlots = 2 };
+int allow_smem(const void* fn, int slot) {
+  static std::atomic<unsigned long long> done[kSlots];  // a bit per device
+  int dev = 0;
+  XAC_CUDA(cudaGetDevice(&dev));
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (bit && (done[slot].load() & bit)) return XAC_OK;
+  XAC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
+  done[slot].fetch_or(bit);
+  return XAC_OK;
+}
+
+// TMA map of a packed BF16 tensor (innermost dimension first), read in boxes whose innermost extent is the swizzle span
+// (128, 64 or 32 bytes). The encoder comes from the driver, once.
+int bf16_map(CUtensorMap* m, const void* base, int rank, const cuuint64_t* dims, const cuuint32_t* box) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                              const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static std::atomic<Encode> fn{nullptr};
+  Encode f = fn.load();
+  if (!f) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    XAC_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q));
+    XAC_REQUIRE(p && q == cudaDriverEntryPointSuccess, "conv3d: the driver has no cuTensorMapEncodeTiled");
+    f = (Encode)p;
+    fn.store(f);
+  }
+  XAC_REQUIRE(((uintptr_t)base & 15u) == 0, "conv3d: operands must be 16-byte aligned");
+  cuuint64_t strides[4];
+  cuuint32_t ones[5] = {1, 1, 1, 1, 1};
+  cuuint64_t bytes = 2;
+  for (int k = 0; k + 1 < rank; ++k) strides[k] = bytes *= dims[k];
+  const CUtensorMapSwizzle sw = box[0] == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : box[0] == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                               : CU_TENSOR_MAP_SWIZZLE_32B;
+  const CUresult e = f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides,
+                       box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  XAC_REQUIRE(e == CUDA_SUCCESS, "conv3d: cuTensorMapEncodeTiled failed (%d)", (int)e);
+  return XAC_OK;
+}
+
+bool search_fwd_plan(const ConvShape& s, int sms, FwdPlan* best) {
+  const int kr = s.ksize / 2, taps = s.ksize * s.ksize * s.ksize;
+  double best_cost = INFINITY;
+  for (int split = 1; split <= s.Co / 16; ++split) {
+    if (s.Co % (16 * split)) continue;
+    const int nb = s.Co / split;
+    const int min_nxt = (s.W + 253) / 254;
+    int last_bx = -1;
+    // x tiles: every count at first, then steps of an eighth, down to tiles of 8 voxels (256 channels need <= 27)
+    for (int nxt = min_nxt; nxt == min_nxt || (s.W + nxt - 1) / nxt >= 8; nxt += nxt < 8 ? 1 : nxt / 8) {
+      const int bx = (s.W + nxt - 1) / nxt, P = bx + 2 * kr;
+      if (bx == last_bx) continue;
+      last_bx = bx;
+      for (int by = 1; by <= s.H; ++by) {
+        const int mt = ((by - 1) * P + bx + kTcM - 1) / kTcM;
+        if (mt * nb > 512 || mt > 2 * kMmaWarps) break;
+        if (P > 256 || by + 2 * kr > 256) break;  // a TMA box
+        const int R = (mt * kTcM + 2 * kr * (P + 1) + 7) / 8 * 8;  // whole swizzle atoms
+        const size_t plane = (size_t)R * s.Ci * 2;
+        if (2 * plane > kSmemLimit) break;
+        for (int ring = 2; ring <= kMaxPlanes; ++ring) {
+          const int march = kr == 1 && ring >= 3;
+          if (kr == 0 && ring == kMaxPlanes) continue;
+          // weights: resident; streamed by taps; streamed by blocks
+          for (int mode = split == 1 ? 0 : 1; mode < 3; ++mode) {
+            const int resident = mode == 0, big = mode < 2;
+            FwdPlan p{};
+            p.KB = 64;
+            while (s.Ci % p.KB) p.KB >>= 1;
+            const int nkc = s.Ci / p.KB;
+            p.G = nkc <= 3 && big ? nkc : 1;
+            if (p.G == 2 && p.KB != 64) p.G = 1;
+            const size_t stage = (size_t)p.KB * p.G * nb * 2;
+            const int stages = taps * (nkc / p.G);
+            p.bs = resident ? stages : kMaxBStages;
+            while (!resident && p.bs > 3 && ring * plane + p.bs * stage > kSmemLimit) --p.bs;
+            p.smem = ring * plane + p.bs * stage;
+            if (p.smem > kSmemLimit) continue;
+            p.bx = bx;
+            p.by = by;
+            p.P = P;
+            p.nxt = (s.W + bx - 1) / bx;
+            p.nyt = (s.H + by - 1) / by;
+            p.mt = mt;
+            p.R = R;
+            p.NS = ring;
+            p.march = march;
+            p.nb = nb;
+            p.nsplit = split;
+            p.resident = resident;
+            p.nbuf = 2 * mt * nb <= 512 ? 2 : 1;
+            p.ncols = 32;
+            while ((int)p.ncols < p.nbuf * mt * nb) p.ncols <<= 1;
+            p.units = (long long)s.N * s.D * p.nyt * p.nxt * split;
+            p.ctas = (int)(p.units < sms ? p.units : sms);
+            const double per = (double)((p.units + p.ctas - 1) / p.ctas);
+            const double hw = 35.0 + nb * 0.24, one = nb / 2.0 > hw ? nb / 2.0 : hw;  // cycles of an MMA
+            // one warp's straight-line issue, and the turn of its loop over stages
+            const int steps = p.KB / 16 * p.G, nt = (mt + kMmaWarps - 1) / kMmaWarps;
+            const double turn = resident && nkc == p.G && kr == 1 ? (steps * nt <= 4 ? 150.0 / 9 : 150.0 / 3) : 250.0;
+            const double issue = 100.0 * steps * nt + turn, stage_hw = mt * one * steps;
+            const double mma = stages * (stage_hw > issue ? stage_hw : issue);
+            const double run = per < s.D ? per : s.D;  // planes of one z walk
+            const double planes = march ? (run + 2) / run : s.ksize;
+            const double bytes = planes * (by + 2 * kr) * P * s.Ci * 2.0 + (resident ? 0.0 : taps * s.Ci * nb * 2.0);
+            const double epi = 300.0 + mt * (nb / 16) * 40.0;
+            const double mem = bytes / 22.0;
+            double unit = mma > mem ? mma + 0.2 * mem : mem + 0.2 * mma;
+            unit = p.nbuf == 2 ? (unit > epi ? unit : epi) + 200.0 : unit + epi + 200.0;
+            const double cost = per * unit + 3000.0 + (resident ? taps * s.Ci * nb * 2.0 / 32.0 : 0.0);
+            if (cost < best_cost) {
+              best_cost = cost;
+              *best = p;
+            }
+          }
+        }
+      }
+    }
+  }
+  return std::isfinite(best_cost);
+}
+
+// Plans kept by shape (the search takes some tens of microseconds); the map is emptied when it holds 256.
+int fwd_plan(const ConvShape& s, FwdPlan* out) {
+  static std::mutex mu;
+  static std::map<std::array<int, 8>, FwdPlan> plans;
+  int sms = 0;
+  int r = sm_count(&sms);
+  if (r != XAC_OK) return r;
+  const std::array<int, 8> key = {s.N, s.D, s.H, s.W, s.Ci, s.Co, s.ksize, sms};
+  try {
+    std::lock_guard<std::mutex> g(mu);
+    auto it = plans.find(key);
+    if (it == plans.end()) {
+      FwdPlan p;
+      XAC_REQUIRE(search_fwd_plan(s, sms, &p), "conv3d: no tile for %d -> %d channels", s.Ci, s.Co);
+      if (plans.size() >= 256) plans.clear();
+      it = plans.emplace(key, p).first;
+    }
+    *out = it->second;
+  } catch (...) {  // no C++ exception crosses the C boundary
+    set_error("conv3d: host allocation failed");
+    return XAC_ENOMEM;
+  }
+  return XAC_OK;
+}
+
 }  // namespace
 }  // namespace xac
 
@@ -486,24 +938,26 @@ int xac_conv3d_forward(const void* in, int N, int D, int H, int W, int Ci, const
   XAC_REQUIRE(in && weight && (out_bf16 || out_f32) && !(out_bf16 && out_f32),
               "xac_conv3d_forward: give exactly one output");
   XAC_REQUIRE(activation == 0 || activation == 1, "xac_conv3d_forward: activation must be 0 (none) or 1 (GELU)");
-  const long long V = (long long)N * D * H * W;
-  TcConv t;
-  t.BK = 64;
-  while (Ci % t.BK != 0) t.BK -= 16;  // 64, 48, 32 or 16
-  t.kt = (ksize == 3 ? 27 : 1) * (Ci / t.BK);
-  t.ncols = 32;
-  while ((int)t.ncols < Co) t.ncols <<= 1;
-  const size_t smem = (size_t)kTcStages * (kTcM + Co) * t.BK * 2;
-  static bool attr_set = false;  // the attribute is per device function; set once per process
-  if (!attr_set) {
-    XAC_CUDA(cudaFuncSetAttribute(conv_fwd_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)((size_t)kTcStages * (kTcM + 256) * 64 * 2)));
-    attr_set = true;
+  FwdPlan pl;
+  r = fwd_plan(s, &pl);
+  if (r != XAC_OK) return r;
+  r = allow_smem((const void*)conv_fwd_kernel, kFwdSlot);
+  if (r != XAC_OK) return r;
+  CUtensorMap tin, tw;
+  const int kr = ksize / 2;
+  {
+    const cuuint64_t dims[5] = {(cuuint64_t)Ci, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N};
+    const cuuint32_t box[5] = {(cuuint32_t)pl.KB, (cuuint32_t)pl.P, (cuuint32_t)(pl.by + 2 * kr), 1, 1};
+    r = bf16_map(&tin, in, 5, dims, box);
+    if (r != XAC_OK) return r;
+    const cuuint32_t taps = (cuuint32_t)(ksize * ksize * ksize);
+    const cuuint64_t wdims[3] = {(cuuint64_t)Ci, (cuuint64_t)Co, taps};
+    const cuuint32_t wbox[3] = {(cuuint32_t)pl.KB, (cuuint32_t)pl.nb, pl.resident ? taps : 1u};
+    r = bf16_map(&tw, weight, 3, wdims, wbox);
+    if (r != XAC_OK) return r;
   }
-  const unsigned grid = (unsigned)((V + kTcM - 1) / kTcM);
-  conv_fwd_tc_kernel<<<grid, 128, smem, as_stream(stream)>>>((const __nv_bfloat16*)in,
-                                                             (const __nv_bfloat16*)weight, bias, s, activation, t,
-                                                             (__nv_bfloat16*)out_bf16, out_f32);
+  conv_fwd_kernel<<<pl.ctas, kFwdThreads, pl.smem, as_stream(stream)>>>(tin, tw, bias, s, activation, pl,
+                                                                        (__nv_bfloat16*)out_bf16, out_f32);
   XAC_CUDA(cudaGetLastError());
   return XAC_OK;
 }
