@@ -325,10 +325,10 @@ typedef struct xac_run_result {
 int xac_lattice_run(xac_lattice *lat, const xac_run_opts *opts, xac_run_result *res, void *stream);
 
 /* ========================================================================== *
- * Warm-start surrogate convolutions: BF16 tensor-core implicit GEMMs (mma.sync m16n8k16), FP32 accumulation.
+ * Warm-start surrogate convolutions: BF16 tensor-core implicit GEMMs (tcgen05), FP32 accumulation.
  * Activations channels-last [N][D][H][W][C] BF16 (DEVICE pointers); weights [taps][Co][Ci] BF16 with
  * taps = 27 (3x3x3, tap = (dz+1)*9 + (dy+1)*3 + (dx+1)) or 1; zero padding; Ci, Co multiples of 16
- * (Ci, Co <= 256). No reference counterpart: the reference's surrogates run through cuDNN
+ * (Ci, Co <= 256); in, weight and d_out on 16-byte boundaries. No reference counterpart: the reference's surrogates run through cuDNN
  * (benchmark/models/unet3d.py:11-125).
  * ========================================================================== */
 /* out = act(bias + conv(in, w)); activation 0 = none, 1 = GELU; exactly one of out_bf16 / out_f32. The data

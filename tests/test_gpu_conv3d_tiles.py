@@ -1,4 +1,4 @@
-"""The forward convolution at the edges of its tiling rule, against torch's FP32 conv3d on the same BF16 operands."""
+"""The convolution kernels at the edges of their tiling rules, against torch on the same BF16 operands."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -40,3 +40,35 @@ def test_forward_tiles(cuda, shape):
     if H > 4:
         part = S.conv_forward(x[:, :, :H - 2].contiguous(), w, b, k, out_fp32=True)
         assert torch.equal(part[:, :, :H - 3], y[:, :, :H - 3])
+
+
+GRAD_SHAPES = [
+    (1, 1, 1, 1, 16, 16, 3),        # one voxel
+    (2, 3, 9, 300, 32, 48, 3),      # rows wider than a tile: d_out copied row by row, its halo columns zero
+    (1, 2, 5, 300, 32, 48, 1),
+    (1, 4, 70, 9, 16, 32, 3),       # three dx taps in M = 128, columns taller than a tile
+    (1, 9, 11, 20, 48, 16, 3),      # three dx taps in M = 64, input channels in blocks
+    (1, 5, 8, 13, 64, 64, 3),       # two dx taps in M = 128 and one in M = 64
+    (1, 3, 6, 10, 128, 144, 3),     # output channels in a block of 128 and one of 16
+    (1, 2, 3, 5, 256, 256, 3),
+    (2, 12, 21, 19, 80, 96, 1),
+]
+
+
+@pytest.mark.parametrize("shape", GRAD_SHAPES)
+def test_weight_grad_tiles(cuda, shape):
+    N, D, H, W, Ci, Co, k = shape
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn((N, D, H, W, Ci), generator=g).cuda().to(S.BF16)
+    dy = torch.randn((N, D, H, W, Co), generator=g).cuda().to(S.BF16)
+    dw, db = S.conv_weight_grad(x, dy, k, True)
+    assert S.kernel_status() == 0
+    xp, d2 = F.pad(x.double(), (0, 0, 1, 1, 1, 1, 1, 1)), dy.double().reshape(-1, Co)
+    # an accumulator takes at most 256 truncating additions (2^-23 of the running sum each), 3e-5 of the sum of
+    # magnitudes at worst; that sum is near 0.64 per voxel against maxima near 4.5 * 4.5
+    tol = 1e-6 * x.float().abs().amax().item() * dy.float().abs().amax().item() * N * D * H * W
+    for t in range(k ** 3):
+        z, r, c = (t // 9, t // 3 % 3, t % 3) if k == 3 else (1, 1, 1)
+        ref = d2.T @ xp[:, z:z + D, r:r + H, c:c + W].reshape(-1, Ci)
+        assert (dw[t] - ref).abs().max().item() <= tol, t
+    assert (db - d2.sum(0)).abs().max().item() <= 1e-6 * dy.float().abs().amax().item() * N * D * H * W

@@ -37,32 +37,8 @@ struct ConvShape {
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 
-// voxel index -> (n, z, y, x); returns the neighbour voxel index for tap offsets, or -1 outside the volume
-struct VoxelCoord {
-  int n, z, y, x;
-};
-// volumes stay below 2^31 voxels (checked on the host): 32-bit decoding
-__device__ __forceinline__ VoxelCoord decode(long long v, const ConvShape& s) {
-  VoxelCoord c;
-  const unsigned u = (unsigned)v, W = (unsigned)s.W, H = (unsigned)s.H, D = (unsigned)s.D;
-  unsigned t = u / W;
-  c.x = (int)(u - t * W);
-  unsigned t2 = t / H;
-  c.y = (int)(t - t2 * H);
-  t = t2 / D;
-  c.z = (int)(t2 - t * D);
-  c.n = (int)t;
-  return c;
-}
-__device__ __forceinline__ long long neighbour(const VoxelCoord& c, int dz, int dy, int dx, const ConvShape& s) {
-  const int z = c.z + dz, y = c.y + dy, x = c.x + dx;
-  if (z < 0 || z >= s.D || y < 0 || y >= s.H || x < 0 || x >= s.W) return -1;
-  return (((long long)c.n * s.D + z) * s.H + y) * s.W + x;
-}
-
 // ---- shared pieces of the tcgen05 kernels ----------------------------------------------------------------
 constexpr int kTcM = 128;
-constexpr int kTcStages = 4;
 constexpr uint32_t kTcSpin = 1u << 22;
 __device__ unsigned int g_conv_status;  // bit 0: a wait ran out
 
@@ -122,14 +98,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -151,9 +119,6 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t alo, uint32_t a
       "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 a, {%1, %2};\n\t"
       "mov.b64 b, {%3, %4};\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
       ::"r"(tmem_d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accum));
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
-  tc_mma(tmem_d, (uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32), idesc, accum);
 }
 // one lane of a converged warp, the same one each time; the compiler then knows that the code under it runs in a
 // single thread and keeps the MMA operands in uniform registers without a loop around every instruction
@@ -571,181 +536,371 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
 }
 
 // ---- weight grad on the tensor cores (tcgen05) --------------------------------------------------------
-// With u = v + off(tap): dw[tap][co][ci] = sum_u d_out[u - off(tap)][co] * in[u][ci], a GEMM with rows
-// m = tap * Co + co (M = taps * Co), columns ci (N = Ci) and K = voxels. A CTA computes 128 rows x Ci columns in
-// tensor memory over one chunk of kWgKC voxels (split K), 64 voxels per stage:
-//   A (MN-major): A[m][u] = d_out[u - off(tap)][co], zero where u - off(tap) leaves the volume;
-//   B (MN-major): B[u][ci] = in[u][ci].
-// Shared-memory layout of both: core matrices of 8 M (or N) values x 8 voxels, 128 contiguous bytes each (one
-// voxel's 8 values per 16-byte row); M/N groups 128 bytes apart (stride byte offset), 8-voxel groups one group
-// row apart (leading byte offset). The chunk's partial goes to partial[chunk][m][ci]; the chunks are added in
-// order by wgrad_reduce_kernel (deterministic). Bounded waits as in the forward kernel.
-constexpr int kWgKC = 4096;  // voxels per CTA
-constexpr int kWgBK = 64;    // voxels per stage
+// dw[tap][co][ci] = sum_v d_out[v][co] * in[v + off(tap)][ci]: GEMMs with K = voxels. Bound: the operands' reads from
+// shared memory (32 bytes per M row and per N column for 16 voxels, 128 B/clk). The kernel before this one gathered d_out
+// from L2 once per tap and voxel; here a tile of d_out and its input planes are copied once by TMA, and every tap is
+// another start address in them:
+//
+//   * A unit is a tile of bx x by voxels of one z plane, as in the forward kernel: d_out's rows r = y*P + x (P = bx + 2;
+//     the two columns after the tile and the rows around it are zeros), the input's three planes with their halo. Both lie
+//     in shared memory as [rows][KB channels] with the row-size swizzle, which is the MN-major layout with K = rows.
+//   * MMA step: 16 rows. B holds the three dy taps of a block of KBx input channels: N groups P rows apart, N = 3 KBx.
+//     A holds up to three dx taps: M groups of KBd output channels one row apart (D[k + g] against X[k + s] is tap dx =
+//     s - g), so 16 output channels fill M = 64 and 32 fill M = 128; 64 channels take two dx taps in M = 128 and the third
+//     in M = 64; more take one.
+//   * One accumulator of a (dz, dx set) is an `Au`. blockIdx.y selects a set of them that fits the 512 columns,
+//     blockIdx.z the block of input channels and of at most 128 output channels, blockIdx.x a range of units.
+//   * Rounding: an accumulator takes at most 256 steps (4096 rows) before it is added, in FP32 on the CUDA cores, to the
+//     CTA's partial in global memory (the tensor core's own additions truncate); wgrad_reduce_kernel adds the partials
+//     of the CTAs in a fixed order.
+//
+// Measured on a B200 with the reductions and db, the kernels before -> these, batch 4: 16 -> 16 channels at 32x128x152
+// 1327 -> 97 us, 48 -> 16 1777 -> 215, 32 -> 32 at 16x64x76 428 -> 43, 192 -> 64 at 8x32x38 259 -> 62; relative error against
+// 64-bit sums 4.8e-6 -> 4.0e-6, 4.7e-6 -> 4.2e-6, 4.7e-6 -> 2.4e-6, 4.2e-6 -> 2.6e-6.
+//
+// Roles: warps 0-7 epilogue, 8-11 MMAs (Au a on warp 8 + a % 4), 12 copies. Waits are bounded as in the forward kernel.
+constexpr int kWgThreads = 416;
+constexpr int kWgEpiWarps = 8;
+constexpr int kWgMaxSteps = 256;  // MMA steps of an accumulator before it is flushed
+constexpr int kWgMaxAu = 9;
+constexpr int kWgLead = 8;  // zero rows before d_out's tile
 
-__global__ void __launch_bounds__(128, 1) conv_wgrad_tc_kernel(const __nv_bfloat16* __restrict__ in,
-                                                               const __nv_bfloat16* __restrict__ dout, ConvShape s,
-                                                               uint32_t ncols, float* __restrict__ partial) {
+struct Au {
+  int dz;   // plane
+  int M;    // 64 or 128
+  int dx0;  // dx tap of M group 0; group g is dx0 - g
+  int ndx;  // dx taps held
+};
+struct WgPlan {
+  int bx, by, P, nxt, nyt;
+  int rows_mode;  // 1: d_out is copied row by row (the tile is narrower than the volume: its halo stays zero)
+  int RX, RD;     // rows of a stored input plane / d_out tile block
+  int NX, march;  // input planes in the ring; 1: kept from one z to the next
+  int KBx, KBd, cb, nblk, mblk;  // channels of a block; output channels of a CTA; blocks of Ci; of Co
+  int nstack;     // dy taps in N
+  int nau, ngr, first[kWgMaxAu + 1];
+  Au au[kWgMaxAu];
+  int nsteps, upc, nbuf;  // steps of a unit, units of an accumulation, accumulator buffers
+  uint32_t ncols;
+  long long units;
+  int ctas;
+  size_t smem;
+};
+
+struct WgBars {
+  uint32_t b0;
+  __device__ __forceinline__ uint32_t xfull(int i) const { return b0 + 8u * i; }
+  __device__ __forceinline__ uint32_t xempty(int i) const { return b0 + 8u * (kMaxPlanes + i); }
+  __device__ __forceinline__ uint32_t dfull(int i) const { return b0 + 8u * (2 * kMaxPlanes + i); }
+  __device__ __forceinline__ uint32_t dempty(int i) const { return b0 + 8u * (2 * kMaxPlanes + 2 + i); }
+  __device__ __forceinline__ uint32_t cfull(int i) const { return b0 + 8u * (2 * kMaxPlanes + 4 + i); }
+  __device__ __forceinline__ uint32_t cempty(int i) const { return b0 + 8u * (2 * kMaxPlanes + 6 + i); }
+  __device__ __forceinline__ uint32_t done() const { return b0 + 8u * (2 * kMaxPlanes + 8); }
+  static constexpr int kCount = 2 * kMaxPlanes + 9;
+};
+
+__host__ __device__ constexpr uint32_t swizzle_of(int kb) {
+  return kb == 64 ? kSwizzle128 : (kb == 32 ? kSwizzle64 : kSwizzle32);
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1) conv_wgrad_kernel(const __grid_constant__ CUtensorMap tin,
+                                                                   const __grid_constant__ CUtensorMap tdo, ConvShape s,
+                                                                   const __grid_constant__ WgPlan pl,
+                                                                   float* __restrict__ partial) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[2 * kTcStages + 1];
+  __shared__ __align__(8) uint64_t bars[WgBars::kCount];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int Ci = s.Ci, Co = s.Co, taps = s.ksize == 3 ? 27 : 1, Mtot = taps * Co;
-  const long long V = (long long)s.N * s.D * s.H * s.W;
-  const int m0 = blockIdx.x * kTcM;
-  const long long u_begin = (long long)blockIdx.y * kWgKC;
-  const long long u_left = V - u_begin;
-  const int KT = (int)(((u_left < kWgKC ? u_left : kWgKC) + kWgBK - 1) / kWgBK);
-  const uint32_t a_bytes = kTcM * kWgBK * 2, b_bytes = (uint32_t)kWgBK * Ci * 2, stage_bytes = a_bytes + b_bytes;
-  const uint32_t a_lbo = (kTcM / 8) * 128u, b_lbo = (uint32_t)(Ci / 8) * 128u;
-  const uint32_t sbase = smem_addr(smem);
-  const uint32_t bar0 = smem_addr(bars);
-  auto full = [&](int st) { return bar0 + 8u * st; };
-  auto empty = [&](int st) { return bar0 + 8u * (kTcStages + st); };
-  const uint32_t done_bar = bar0 + 8u * (2 * kTcStages);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int kr = s.ksize >> 1, nd = s.ksize, taps = nd * nd * nd, P = pl.P, D = s.D;
+  const int blk = blockIdx.z % pl.nblk, m0 = (int)(blockIdx.z / pl.nblk) * 128;
+  const int cb = s.Co - m0 < pl.cb ? s.Co - m0 : pl.cb, ndb = cb / pl.KBd;  // this CTA's output channels, in blocks
+  const int au0 = pl.first[blockIdx.y], au1 = pl.first[blockIdx.y + 1];
+  const int dlo = pl.au[au0].dz, ndz = pl.au[au1 - 1].dz - dlo + 1;  // planes used
+  const int N = pl.KBx * pl.nstack, naus = au1 - au0;
+  const int nmw = naus < kMmaWarps ? naus : kMmaWarps;
+  const uint32_t xrow = (uint32_t)pl.KBx * 2u, drow = (uint32_t)pl.KBd * 2u;
+  const uint32_t dslot = (uint32_t)(pl.cb / pl.KBd) * pl.RD * drow, xslot = (uint32_t)pl.RX * xrow;
+  const uint32_t d0 = smem_addr(smem), x0 = d0 + 2u * dslot;
+  const WgBars bar{smem_addr(bars)};
+
+  // rows that no copy writes (before, between and after the tiles) are read against zeros: they must be finite
+  for (uint32_t i = tid * 16u; i < (uint32_t)pl.smem; i += kWgThreads * 16u)
+    *reinterpret_cast<uint4*>(smem + i) = make_uint4(0u, 0u, 0u, 0u);
+  fence_proxy_async();
   if (tid == 0) {
-    for (int st = 0; st < kTcStages; ++st) {
-      mbar_init(full(st), 128);
-      mbar_init(empty(st), 1);
+    for (int i = 0; i < kMaxPlanes; ++i) {
+      mbar_init(bar.xfull(i), 1);
+      mbar_init(bar.xempty(i), nmw);
     }
-    mbar_init(done_bar, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar.dfull(i), 1);
+      mbar_init(bar.dempty(i), nmw);
+      mbar_init(bar.cfull(i), nmw);
+      mbar_init(bar.cempty(i), 32 * kWgEpiWarps);
+    }
+    mbar_init(bar.done(), nmw);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
-                 "r"(ncols));
+                 "r"(pl.ncols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const uint32_t idesc = tc_idesc(Ci) | (1u << 15) | (1u << 16);  // A and B MN-major
-  const int ul = tid & 63, g0 = tid >> 6;  // this thread's voxel in a stage, and first M / N group
-  const int kg = ul >> 3, krow = ul & 7;
-
-  auto load_stage = [&](int k, int st) {
-    const uint32_t a_st = sbase + (uint32_t)st * stage_bytes, b_st = a_st + a_bytes;
-    const long long u = u_begin + (long long)k * kWgBK + ul;
-    const bool uok = u < V && k * kWgBK + ul < kWgKC;
-    const VoxelCoord cu = decode(uok ? u : 0, s);
-    for (int j = 0; j < 8; ++j) {
-      const int mg = g0 + 2 * j, m = m0 + mg * 8;
-      long long src = -1;
-      int co = 0;
-      if (uok && m < Mtot) {
-        const int tap = m / Co;
-        co = m - tap * Co;
-        const int dz = s.ksize == 3 ? tap / 9 - 1 : 0, dy = s.ksize == 3 ? (tap / 3) % 3 - 1 : 0,
-                  dx = s.ksize == 3 ? tap % 3 - 1 : 0;
-        src = neighbour(cu, -dz, -dy, -dx, s);
-      }
-      cp_async16(a_st + ((uint32_t)(kg * (kTcM / 8) + mg) * 8u + krow) * 16u,
-                 src >= 0 ? (const void*)(dout + src * Co + co) : (const void*)dout, src >= 0 ? 16u : 0u);
-    }
-    for (int ng = g0; ng < Ci / 8; ng += 2)
-      cp_async16(b_st + ((uint32_t)(kg * (Ci / 8) + ng) * 8u + krow) * 16u,
-                 uok ? (const void*)(in + u * Ci + ng * 8) : (const void*)in, uok ? 16u : 0u);
+  volatile int* abort_v = &abort_flag;
+  const long long u_begin = pl.units * blockIdx.x / gridDim.x, u_end = pl.units * (blockIdx.x + 1) / gridDim.x;
+  // unit = ((n * nyt + y tile) * nxt + x tile) * D + z
+  struct Tile {
+    int n, y0, x0;
   };
-  auto mma_stage = [&](int k, int st) {
-    const uint32_t a_st = sbase + (uint32_t)st * stage_bytes, b_st = a_st + a_bytes;
-    for (int q = 0; q < kWgBK / 16; ++q) {
-      const uint64_t ad = smem_desc(a_st + (uint32_t)(2 * q) * a_lbo, a_lbo, 128u);
-      const uint64_t bd = smem_desc(b_st + (uint32_t)(2 * q) * b_lbo, b_lbo, 128u);
-      tc_mma(tmem, ad, bd, idesc, (k > 0 || q > 0) ? 1u : 0u);
-    }
-    tc_commit(empty(st));
+  auto tile_of = [&](long long strip) {
+    Tile t;
+    unsigned v = (unsigned)strip;
+    t.x0 = (int)(v % pl.nxt) * pl.bx;
+    v /= pl.nxt;
+    t.y0 = (int)(v % pl.nyt) * pl.by;
+    t.n = (int)(v / pl.nyt);
+    return t;
   };
 
-  for (int k = 0; k < KT + kTcStages - 1; ++k) {
-    if (k < KT) {
-      const int st = k % kTcStages;
-      if (k >= kTcStages && !mbar_wait(empty(st), ((k / kTcStages) - 1) & 1)) abort_flag = 1;
-      if (abort_flag) break;
-      load_stage(k, st);
-    }
-    cp_async_commit();
-    const int kc = k - (kTcStages - 1);
-    if (kc >= 0) {
-      cp_async_wait<kTcStages - 1>();
-      fence_proxy_async();
-      mbar_arrive(full(kc % kTcStages));
-      if (warp == 0) {
-        if (mbar_wait(full(kc % kTcStages), (kc / kTcStages) & 1)) {
-          tc_fence_after();
-          if (lane == 0) mma_stage(kc, kc % kTcStages);
-        } else {
-          abort_flag = 1;
+  if (warp == kWgEpiWarps + kMmaWarps) {
+    if (lane == 0) {
+      const uint32_t xbytes = (uint32_t)(P * (pl.by + 2 * kr)) * xrow;
+      const uint32_t dbytes = (uint32_t)(ndb * pl.by * (pl.rows_mode ? pl.bx : P)) * drow;
+      int xs = 0, ds = 0, xseq = 0, dseq = 0;
+      uint32_t xpar = 1, dpar = 1;
+      auto load_x = [&](const Tile& t, int z) -> bool {
+        if (!mbar_wait_or_abort(bar.xempty(xs), xpar, abort_v)) return false;
+        mbar_expect_tx(bar.xfull(xs), xbytes);
+        tma_load_5d(x0 + (uint32_t)xs * xslot, &tin, blk * pl.KBx, t.x0 - kr, t.y0 - kr, z, t.n, bar.xfull(xs));
+        ++xseq;
+        if (++xs == pl.NX) {
+          xs = 0;
+          xpar ^= 1u;
         }
-        __syncwarp();
+        return true;
+      };
+      auto load_d = [&](const Tile& t, int z) -> bool {
+        if (!mbar_wait_or_abort(bar.dempty(ds), dpar, abort_v)) return false;
+        mbar_expect_tx(bar.dfull(ds), dbytes);
+        for (int k = 0; k < ndb; ++k) {
+          const uint32_t dst = d0 + (uint32_t)ds * dslot + (uint32_t)(k * pl.RD + kWgLead) * drow;
+          if (pl.rows_mode) {
+            for (int y = 0; y < pl.by; ++y)
+              tma_load_5d(dst + (uint32_t)(y * P) * drow, &tdo, m0 + k * pl.KBd, t.x0, t.y0 + y, z, t.n, bar.dfull(ds));
+          } else {
+            tma_load_5d(dst, &tdo, m0 + k * pl.KBd, 0, t.y0, z, t.n, bar.dfull(ds));
+          }
+        }
+        ++dseq;
+        if (++ds == 2) {
+          ds = 0;
+          dpar ^= 1u;
+        }
+        return true;
+      };
+      bool ok = true;
+      for (long long u = u_begin; ok && u < u_end;) {
+        const long long strip = u / D;
+        const int z0 = (int)(u - strip * D);
+        const int nz = (int)((u_end - u < D - z0) ? u_end - u : D - z0);
+        const Tile t = tile_of(strip);
+        for (int i = 0; ok && i < nz; ++i) {
+          ok = load_d(t, z0 + i);
+          for (int d = (pl.march && i > 0) ? ndz - 1 : 0; ok && d < ndz; ++d) ok = load_x(t, z0 + i + dlo + d - kr);
+        }
+        u += nz;
+      }
+      // an abort may leave copies that no role waited for: let them land before the block's memory goes back
+      if (*abort_v) {
+        for (int k = xseq > pl.NX ? xseq - pl.NX : 0; k < xseq; ++k) mbar_wait(bar.xfull(k % pl.NX), (k / pl.NX) & 1);
+        for (int k = dseq > 2 ? dseq - 2 : 0; k < dseq; ++k) mbar_wait(bar.dfull(k & 1), (k >> 1) & 1);
       }
     }
-    if (abort_flag) break;
-  }
-  cp_async_wait<0>();
-  if (tid == 0) tc_commit(done_bar);
-  const int drained = mbar_wait(done_bar, 0) ? 1 : 0;
-  const bool ok = __syncthreads_and(drained) && !abort_flag;
-  tc_fence_after();
-  if (ok) {
-    const int m = m0 + warp * 32 + lane;
-    float* dst = partial + ((long long)blockIdx.y * Mtot + m) * Ci;
-    for (int c0 = 0; c0 < Ci; c0 += 16) {
-      float x[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, x);
-      if (m < Mtot) {
-        float4* d4 = reinterpret_cast<float4*>(dst + c0);
+  } else if (warp >= kWgEpiWarps) {
+    const int t0 = warp - kWgEpiWarps;
+    if (t0 < nmw) {
+      // SBO: the next 8 rows; LBO: the next M / N group (one row on where it is another dx tap, a block on otherwise)
+      const uint64_t ad = smem_desc(d0, ndb == 1 ? drow : (uint32_t)pl.RD * drow, 8u * drow) |
+                          ((uint64_t)swizzle_of(pl.KBd) << 61);
+      const uint64_t bd = smem_desc(x0, (uint32_t)P * xrow, 8u * xrow) | ((uint64_t)swizzle_of(pl.KBx) << 61);
+      const uint32_t ahi = (uint32_t)(ad >> 32), bhi = (uint32_t)(bd >> 32);
+      const uint32_t astep = drow, bstep = xrow;  // 16 rows in 16-byte units
+      const int issuer = elect_one() ? 1 : 0;
+      int cnt = 0, buf = 0, ds = 0, xseq0 = 0, unit = 0;
+      uint32_t dpar = 0;
+      bool ok = true;
+      for (long long u = u_begin; ok && u < u_end;) {
+        const int z0 = (int)(u % D);
+        const int nz = (int)((u_end - u < D - z0) ? u_end - u : D - z0);
+        for (int i = 0; ok && i < nz; ++i, ++unit) {
+          const bool first = unit % pl.upc == 0, last = unit % pl.upc == pl.upc - 1 || u + i == u_end - 1;
+          if (first) {
+            buf = cnt % pl.nbuf;
+            if (cnt >= pl.nbuf && !mbar_wait_or_abort(bar.cempty(buf), ((cnt / pl.nbuf) - 1) & 1, abort_v)) ok = false;
+            ++cnt;
+          }
+          if (ok) ok = mbar_wait_or_abort(bar.dfull(ds), dpar, abort_v);
+          for (int d = 0; ok && d < ndz; ++d) {
+            const int sq = xseq0 + (pl.march ? i + d : i * ndz + d), slot = sq % pl.NX;
+            if (!mbar_wait_or_abort(bar.xfull(slot), (sq / pl.NX) & 1, abort_v)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            if (issuer) {
+              for (int a = t0; a < naus; a += kMmaWarps) {
+                const Au& au = pl.au[au0 + a];
+                if (au.dz != dlo + d) continue;
+                const uint32_t idesc = (tc_idesc(N) & ~(31u << 24)) | ((uint32_t)(au.M >> 4) << 24) | (1u << 15) | (1u << 16);
+                const uint32_t acc = tmem + (uint32_t)((buf * naus + a) * N);
+                // M group g reads D[k + g] with X[k + dx0]: k starts at -(ndx - 1)
+                uint32_t alo = (uint32_t)ad + ((uint32_t)ds * dslot + (uint32_t)(kWgLead - (au.ndx - 1)) * drow) / 16u;
+                uint32_t blo = (uint32_t)bd + ((uint32_t)slot * xslot + (uint32_t)(au.dx0 - (au.ndx - 1)) * xrow) / 16u;
+                uint32_t accum = first ? 0u : 1u;
+#pragma unroll 2
+                for (int j = 0; j < pl.nsteps; j += 4) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) d4[i] = make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+                  for (int k = 0; k < 4; ++k) {
+                    tc_mma(acc, alo + (uint32_t)k * astep, ahi, blo + (uint32_t)k * bstep, bhi, idesc, accum);
+                    accum = 1u;
+                  }
+                  alo += 4u * astep;
+                  blo += 4u * bstep;
+                }
+              }
+              if (!pl.march || d == 0 || i == nz - 1) tc_commit(bar.xempty(slot));
+            }
+            __syncwarp();
+          }
+          if (ok && issuer) {
+            tc_commit(bar.dempty(ds));
+            if (last) tc_commit(bar.cfull(buf));
+          }
+          __syncwarp();
+          ds ^= 1;
+          if (ds == 0) dpar ^= 1u;
+        }
+        xseq0 += pl.march ? nz + ndz - 1 : nz * ndz;
+        u += nz;
       }
+      if (issuer) tc_commit(bar.done());
+    }
+  } else {
+    // ---- flush: accumulator rows of M = 64 lie in the first 16 lanes of each warp quadrant, of M = 128 in all 32
+    const int quad = warp & 3, groups = N >> 4;
+    const long long nu = u_end - u_begin;
+    const int flushes = (int)((nu + pl.upc - 1) / pl.upc);
+    float* base = partial + (long long)blockIdx.x * taps * s.Co * s.Ci;
+    for (int f = 0; f < flushes; ++f) {
+      const int buf = f % pl.nbuf;
+      if (!mbar_wait_or_abort(bar.cfull(buf), (f / pl.nbuf) & 1, abort_v)) break;
+      tc_fence_after();
+      for (int it = warp >> 2; it < naus * groups; it += kWgEpiWarps / 4) {
+        const int a = it / groups, c0 = (it - a * groups) << 4;
+        const Au& au = pl.au[au0 + a];
+        float v[16];
+        __syncwarp();
+        tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)((buf * naus + a) * N + c0), v);
+        const int m = au.M == 64 ? quad * 16 + lane : quad * 32 + lane;
+        const int g = ndb == 1 ? m / pl.KBd : 0, co = ndb == 1 ? m - g * pl.KBd : m;
+        if (au.M == 64 && lane >= 16) continue;
+        if (g >= au.ndx || co >= cb) continue;
+        const int dy = c0 / pl.KBx, ci = blk * pl.KBx + c0 - dy * pl.KBx;
+        const int tap = nd == 3 ? au.dz * 9 + dy * 3 + au.dx0 - g : 0;
+        float4* dst = reinterpret_cast<float4*>(base + ((long long)tap * s.Co + m0 + co) * s.Ci + ci);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float4 p = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          if (f > 0) {
+            const float4 o = dst[i];
+            p = make_float4(o.x + p.x, o.y + p.y, o.z + p.z, o.w + p.w);
+          }
+          dst[i] = p;
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(bar.cempty(buf));
     }
   }
-  tc_fence_before();
+  __syncwarp();
+  mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(pl.ncols));
   }
 }
 
-// dw[t][co][ci] = sum over chunks in order; db[co] = sum of d_out over voxels (block per co, fixed order)
-__global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int nchunks, long long per_chunk,
-                                    float* __restrict__ dw) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= per_chunk) return;
-  float s = 0.0f;
-  for (int k = 0; k < nchunks; ++k) s += partial[(long long)k * per_chunk + e];
-  dw[e] = s;
-}
-
-// db[co] = sum over voxels of d_out: 256 blocks stride over voxels (consecutive threads read consecutive channels),
-// each block reduces its channel sums in a fixed order into one partial row, a second pass adds the rows in order
-constexpr int kBiasBlocks = 256;
-__global__ void bias_grad_partial_kernel(const __nv_bfloat16* __restrict__ dout, long long V, int Co,
-                                         float* __restrict__ partial) {
-  __shared__ float part[256];
-  const int c = threadIdx.x % Co, lanes = blockDim.x / Co, g = threadIdx.x / Co;
-  float s = 0.0f;
-  if (g < lanes)
-    for (long long v = (long long)blockIdx.x * lanes + g; v < V; v += (long long)gridDim.x * lanes)
-      s += __bfloat162float(dout[v * Co + c]);
-  part[threadIdx.x] = s;
+// db[co] = sum over voxels of d_out. Bound: one read of d_out. A thread takes 8 channels (16 bytes) of every
+// stride-th voxel; the block's sums per channel go to one row of partials, which a second pass adds in order.
+constexpr int kBiasBlocks = 592;
+__global__ void __launch_bounds__(256) bias_grad_partial_kernel(const __nv_bfloat16* __restrict__ dout, long long V, int Co,
+                                                                float* __restrict__ partial) {
+  __shared__ float part[256][9];
+  const int oct = Co >> 3, lanes = 256 / oct, o = threadIdx.x % oct, g = threadIdx.x / oct;
+  float a[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  if (g < lanes) {
+    const uint4* src = reinterpret_cast<const uint4*>(dout) + o;
+#pragma unroll 4
+    for (long long v = (long long)blockIdx.x * lanes + g; v < V; v += (long long)gridDim.x * lanes) {
+      const uint4 q = __ldg(src + v * oct);
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[2 * i] += __uint_as_float(w[i] << 16);
+        a[2 * i + 1] += __uint_as_float(w[i] & 0xffff0000u);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) part[threadIdx.x][i] = a[i];
   __syncthreads();
   if ((int)threadIdx.x < Co) {
+    const int co = threadIdx.x;
     float t = 0.0f;
-    for (int k = 0; k < lanes; ++k) t += part[k * Co + threadIdx.x];
-    partial[(long long)blockIdx.x * Co + threadIdx.x] = t;
+    for (int k = 0; k < lanes; ++k) t += part[k * oct + (co >> 3)][co & 7];
+    partial[(long long)blockIdx.x * Co + co] = t;
   }
 }
 
-__global__ void bias_grad_final_kernel(const float* __restrict__ partial, int nblocks, int Co, float* __restrict__ db) {
-  const int c = threadIdx.x;
-  if (c >= Co) return;
+// The partial sums of both, one launch. dw[e] = sum of the CTAs' partials: a block sums 32 values, 8 segments of the CTAs
+// each in order, then the segments in order. The blocks after those take db: a warp per channel, 32 strided sums
+// of the bias partials, then a fixed tree.
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, int n, long long count,
+                                                           float* __restrict__ dw, const float* __restrict__ bias_partial,
+                                                           int bias_rows, int Co, float* __restrict__ db) {
+  __shared__ float part[8][33];
+  const int x = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const long long dw_blocks = (count + 31) / 32;
+  if (blockIdx.x >= dw_blocks) {
+    const int c = (int)(blockIdx.x - dw_blocks) * 8 + seg;
+    if (c >= Co) return;
+    float t = 0.0f;
+    for (int b = x; b < bias_rows; b += 32) t += bias_partial[(long long)b * Co + c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (x == 0) db[c] = t;
+    return;
+  }
+  const long long e = blockIdx.x * 32ll + x;
   float t = 0.0f;
-  for (int b = 0; b < nblocks; ++b) t += partial[(long long)b * Co + c];
-  db[c] = t;
+  if (e < count) {
+    const int k0 = n * seg / 8, k1 = n * (seg + 1) / 8;
+#pragma unroll 8
+    for (int k = k0; k < k1; ++k) t += partial[(long long)k * count + e];
+  }
+  part[seg][x] = t;
+  __syncthreads();
+  if (seg == 0 && e < count) {
+    for (int k = 1; k < 8; ++k) t += part[k][x];
+    dw[e] = t;
+  }
 }
 
 int check_shape(const ConvShape& s) {
@@ -923,6 +1078,126 @@ int fwd_plan(const ConvShape& s, FwdPlan* out) {
   return XAC_OK;
 }
 
+// ---- host: the weight gradient's tile ---------------------------------------------------------------------------
+// A pure function of the shape (148 CTAs are assumed, whatever the device: the partial buffer's size is part of the ABI).
+constexpr int kWgCtas = 148;
+
+bool search_wg_plan(const ConvShape& s, WgPlan* best) {
+  const int kr = s.ksize / 2, nd = s.ksize;
+  WgPlan b{};
+  b.KBx = b.KBd = 64;
+  while (s.Ci % b.KBx) b.KBx >>= 1;
+  while (s.Co % b.KBd) b.KBd >>= 1;
+  b.nblk = s.Ci / b.KBx;
+  b.cb = s.Co < 128 ? s.Co : 128;
+  b.mblk = (s.Co + 127) / 128;
+  b.nstack = nd;
+  const int N = b.KBx * b.nstack, M1 = s.Co <= 64 ? 64 : 128;
+  for (int dz = 0; dz < nd; ++dz) {
+    if (nd == 1) {
+      b.au[b.nau++] = {0, M1, 0, 1};
+    } else if (s.Co == 16 || s.Co == 32) {
+      b.au[b.nau++] = {dz, s.Co == 16 ? 64 : 128, 2, 3};
+    } else if (s.Co == 64) {
+      b.au[b.nau++] = {dz, 128, 2, 2};
+      b.au[b.nau++] = {dz, 64, 0, 1};
+    } else {
+      for (int dx = 0; dx < 3; ++dx) b.au[b.nau++] = {dz, M1, dx, 1};
+    }
+  }
+  // accumulator sets of at most 512 columns, as even as their number allows
+  const int cap = 512 / N;
+  b.ngr = (b.nau + cap - 1) / cap;
+  for (int g = 0; g <= b.ngr; ++g) b.first[g] = b.nau * g / b.ngr;
+  int most = 0, planes = 0;
+  double mma = 0.0;  // cycles of a step, in the longest set
+  for (int g = 0; g < b.ngr; ++g) {
+    const int n = b.first[g + 1] - b.first[g];
+    double c = 0.0;
+    for (int a = b.first[g]; a < b.first[g + 1]; ++a) {
+      const double rd = (b.au[a].M + N) / 4.0 + 8.0, math = N / 2.0;
+      c += rd > math ? rd : math;
+    }
+    const double issue = 60.0 * ((n + kMmaWarps - 1) / kMmaWarps);
+    if (c < issue) c = issue;
+    if (c > mma) mma = c;
+    if (n > most) most = n;
+    const int pz = b.au[b.first[g + 1] - 1].dz - b.au[b.first[g]].dz + 1;
+    if (pz > planes) planes = pz;
+  }
+  b.nbuf = 2 * most * N <= 512 ? 2 : 1;
+  b.ncols = 32;
+  while ((int)b.ncols < b.nbuf * most * N) b.ncols <<= 1;
+  const int sets = b.ngr * b.nblk * b.mblk;
+  double best_cost = INFINITY;
+  const int pitches[] = {0, 256, 128, 64, 48, 32, 24, 16, 8};  // 0: the whole row of the volume
+  for (int pitch : pitches) {
+    WgPlan p = b;
+    p.rows_mode = pitch != 0;
+    p.P = pitch ? pitch : s.W + 2 * kr;
+    p.bx = p.P - 2 * kr;
+    if (p.P > 256 || (pitch && p.bx >= s.W)) continue;
+    p.nxt = (s.W + p.bx - 1) / p.bx;
+    for (p.by = 1; p.by <= s.H && p.by + 2 * kr <= 256; ++p.by) {
+      p.nsteps = ((p.by * p.P + 2 * kr + 15) / 16 + 3) / 4 * 4;
+      if (p.nsteps > kWgMaxSteps) break;
+      // the last step's rows, the farthest M group and dy tap stay inside a block
+      p.RD = (kWgLead + p.nsteps * 16 + 8 + 7) / 8 * 8;
+      p.RX = (p.nsteps * 16 + 2 + 2 * kr * p.P + 7) / 8 * 8;
+      if (p.RX < (p.by + 2 * kr) * p.P) p.RX = ((p.by + 2 * kr) * p.P + 7) / 8 * 8;
+      p.nyt = (s.H + p.by - 1) / p.by;
+      const size_t dtile = (size_t)p.RD * p.cb * 2, plane = (size_t)p.RX * p.KBx * 2;
+      for (p.NX = 2; p.NX <= kMaxPlanes; ++p.NX) {
+        p.march = p.NX > planes || (p.NX == planes && planes == 3);
+        if (planes == 1) p.march = 0;
+        p.smem = 2 * dtile + p.NX * plane;
+        // M groups past the last block read on from the second tile: keep them inside
+        const size_t reach = dtile + (size_t)(128 / p.KBd) * p.RD * p.KBd * 2;
+        if (p.smem < reach) p.smem = reach;
+        if (p.smem > kSmemLimit) break;
+        p.upc = kWgMaxSteps / p.nsteps;
+        p.units = (long long)s.N * s.D * p.nyt * p.nxt;
+        const long long room = kWgCtas / sets > 0 ? kWgCtas / sets : 1;
+        p.ctas = (int)(p.units < room ? p.units : room);
+        const double waves = (double)((p.ctas * sets + kWgCtas - 1) / kWgCtas);
+        const double per = (double)((p.units + p.ctas - 1) / p.ctas), run = per < s.D ? per : s.D;
+        const double loads = p.march ? (run + planes - 1) / run : planes;
+        const double mem = (p.by * p.P * p.cb * 2.0 + loads * (p.by + 2 * kr) * p.P * p.KBx * 2.0) / 22.0;
+        const double work = mma * p.nsteps;
+        const double flush = 500.0 + most * (N / 16) * 60.0;
+        const double unit = (work > mem ? work + 0.2 * mem : mem + 0.2 * work) + 200.0 + (p.nbuf == 1 ? flush / p.upc : 0.0);
+        const double cost = waves * (per * unit + 5000.0 + flush);
+        if (cost < best_cost) {
+          best_cost = cost;
+          *best = p;
+        }
+      }
+    }
+  }
+  return std::isfinite(best_cost);
+}
+
+int wg_plan(const ConvShape& s, WgPlan* out) {
+  static std::mutex mu;
+  static std::map<std::array<int, 7>, WgPlan> plans;
+  const std::array<int, 7> key = {s.N, s.D, s.H, s.W, s.Ci, s.Co, s.ksize};
+  try {
+    std::lock_guard<std::mutex> g(mu);
+    auto it = plans.find(key);
+    if (it == plans.end()) {
+      WgPlan p;
+      XAC_REQUIRE(search_wg_plan(s, &p), "conv3d: no weight-gradient tile for %d -> %d channels", s.Ci, s.Co);
+      if (plans.size() >= 256) plans.clear();
+      it = plans.emplace(key, p).first;
+    }
+    *out = it->second;
+  } catch (...) {  // no C++ exception crosses the C boundary
+    set_error("conv3d: host allocation failed");
+    return XAC_ENOMEM;
+  }
+  return XAC_OK;
+}
+
 }  // namespace
 }  // namespace xac
 
@@ -962,7 +1237,7 @@ int xac_conv3d_forward(const void* in, int N, int D, int H, int W, int Ci, const
   return XAC_OK;
 }
 
-// partial must hold ceil(V / 2048) * taps * Co * Ci floats; dw receives taps * Co * Ci floats, db Co floats
+// partial must hold xac_conv3d_partial_floats() floats; dw receives taps * Co * Ci floats, db Co floats
 int xac_conv3d_weight_grad(const void* in, int N, int D, int H, int W, int Ci, const void* dout, int Co, int ksize,
                            float* partial, float* dw, float* db, void* stream) {
   ConvShape s{N, D, H, W, Ci, Co, ksize};
@@ -970,28 +1245,35 @@ int xac_conv3d_weight_grad(const void* in, int N, int D, int H, int W, int Ci, c
   if (r != XAC_OK) return r;
   XAC_REQUIRE(in && dout && partial && dw, "xac_conv3d_weight_grad: null pointer");
   const long long V = (long long)N * D * H * W;
-  const int taps = ksize == 3 ? 27 : 1;
-  const int nchunks = (int)((V + kWgKC - 1) / kWgKC);
-  uint32_t ncols = 32;
-  while ((int)ncols < Ci) ncols <<= 1;
-  static bool attr_set = false;
-  if (!attr_set) {
-    XAC_CUDA(cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)((size_t)kTcStages * (kTcM * kWgBK + kWgBK * 256) * 2)));
-    attr_set = true;
+  const int taps = ksize == 3 ? 27 : 1, kr = ksize / 2;
+  WgPlan pl;
+  r = wg_plan(s, &pl);
+  if (r != XAC_OK) return r;
+  r = allow_smem((const void*)conv_wgrad_kernel, kWgSlot);
+  if (r != XAC_OK) return r;
+  CUtensorMap tin, tdo;
+  {
+    const cuuint64_t dims[5] = {(cuuint64_t)Ci, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N};
+    const cuuint32_t box[5] = {(cuuint32_t)pl.KBx, (cuuint32_t)pl.P, (cuuint32_t)(pl.by + 2 * kr), 1, 1};
+    r = bf16_map(&tin, in, 5, dims, box);
+    if (r != XAC_OK) return r;
+    const cuuint64_t ddims[5] = {(cuuint64_t)Co, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)N};
+    const cuuint32_t dbox[5] = {(cuuint32_t)pl.KBd, (cuuint32_t)(pl.rows_mode ? pl.bx : pl.P),
+                                (cuuint32_t)(pl.rows_mode ? 1 : pl.by), 1, 1};
+    r = bf16_map(&tdo, dout, 5, ddims, dbox);
+    if (r != XAC_OK) return r;
   }
-  const dim3 grid((unsigned)((taps * Co + kTcM - 1) / kTcM), (unsigned)nchunks);
-  const size_t smem = (size_t)kTcStages * (kTcM * kWgBK + kWgBK * Ci) * 2;
   cudaStream_t st = as_stream(stream);
-  conv_wgrad_tc_kernel<<<grid, 128, smem, st>>>((const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, s, ncols,
-                                                 partial);
-  const long long per_chunk = (long long)taps * Co * Ci;
-  wgrad_reduce_kernel<<<(unsigned)((per_chunk + 255) / 256), 256, 0, st>>>(partial, nchunks, per_chunk, dw);
-  if (db) {
-    // the bias partials reuse the head of `partial` after the weight reduction has consumed it
-    bias_grad_partial_kernel<<<kBiasBlocks, 256, 0, st>>>((const __nv_bfloat16*)dout, V, Co, partial);
-    bias_grad_final_kernel<<<1, Co, 0, st>>>(partial, kBiasBlocks, Co, db);
-  }
+  conv_wgrad_kernel<<<dim3((unsigned)pl.ctas, (unsigned)pl.ngr, (unsigned)(pl.nblk * pl.mblk)), kWgThreads, pl.smem, st>>>(
+      tin, tdo, s, pl, partial);
+  const long long count = (long long)taps * Co * Ci;
+  float* bias_partial = partial + pl.ctas * count;
+  const int lanes = 256 / (Co / 8);
+  const int rows = (int)((V + lanes - 1) / lanes < kBiasBlocks ? (V + lanes - 1) / lanes : kBiasBlocks);
+  if (db)
+    bias_grad_partial_kernel<<<rows, 256, 0, st>>>((const __nv_bfloat16*)dout, V, Co, bias_partial);
+  wgrad_reduce_kernel<<<(unsigned)((count + 31) / 32) + (db ? (Co + 7) / 8 : 0), 256, 0, st>>>(
+      partial, pl.ctas, count, dw, bias_partial, rows, Co, db);
   XAC_CUDA(cudaGetLastError());
   return XAC_OK;
 }
@@ -1032,10 +1314,13 @@ int xac_conv3d_status(int* flags) {
 
 int xac_conv3d_partial_floats(int N, int D, int H, int W, int Ci, int Co, int ksize, long long* count) {
   XAC_REQUIRE(count, "xac_conv3d_partial_floats: null pointer");
-  const long long V = (long long)N * D * H * W;
-  const long long w = ((V + kWgKC - 1) / kWgKC) * (ksize == 3 ? 27 : 1) * (long long)Co * Ci;
-  const long long b = (long long)kBiasBlocks * Co;
-  *count = w > b ? w : b;
+  const ConvShape s{N, D, H, W, Ci, Co, ksize};
+  int r = check_shape(s);
+  if (r != XAC_OK) return r;
+  WgPlan pl;
+  r = wg_plan(s, &pl);
+  if (r != XAC_OK) return r;
+  *count = (long long)pl.ctas * (ksize == 3 ? 27 : 1) * Co * Ci + (long long)kBiasBlocks * Co;
   return XAC_OK;
 }
 
