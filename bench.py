@@ -256,7 +256,7 @@ def run_reference_arm(args):
 
 
 # ------------------------------------------------------------------------------------------------ GPU
-STEP_KERNELS = {0: "coupled_step_kernel<float>", 1: "coupled_qstage_kernel<float>"}
+STEP_KERNELS = {0: "split_fluid_kernel<float> + split_thermal_kernel<float>", 1: "coupled_qstage_kernel<float>"}
 # The first of the benchmark gyroid seeds 0-23 whose cold solve reaches residual 1e-6 within 30000 steps (19,800
 # steps; seed 0 stops at the step limit, 11 of the 24 trip the divergence guard at the first check).
 CONVERGED_SEED = 15
@@ -557,7 +557,7 @@ def run_gpu_arm(args):
                         "solves_s": [round(x, 4) for x in solve_s],
                         "solver_steps": res["steps"], "converged": res["converged"],
                         "converged_design": conv_e2e},
-                "gpu_launches": args.steps * (STEPS_PER_BENCH_STEP + 3),
+                "gpu_launches": args.steps * (STEPS_PER_BENCH_STEP * (2 if shape["variant"] == 0 else 1) + 3),
                 "launch_shape": {"block": shape["block"], "variant": shape["variant"], "autotuned": shape["table"]},
                 "forms": forms,
                 "clocks": clk.summary(),

@@ -228,10 +228,10 @@ int xac_lattice_fields(xac_lattice *lat, float *rho, float *u, float *T, void *s
 int xac_lattice_set_inlet(xac_lattice *lat, double u_inlet, void *stream);
 int xac_lattice_get_inlet(xac_lattice *lat, double *u_inlet, void *stream);
 int xac_lattice_steps_done(const xac_lattice *lat, long long *steps);
-/* Launch shape of the fused step kernel: threads per block (64, 128, 256) and the visiting order:
- * variant 0 = one thread per row position, in memory order; variant 1 = one block per row whose thermal input is
- * staged in shared memory by bulk copies while the fluid lattice runs (row lengths 64..256; other lengths run
- * variant 0). Variant 1 waits for its copies with a bounded wait; if a wait ever gives up, the call that sees it
+/* Launch shape of the step: threads per block (64, 128, 256) and the variant: 0 = the fluid and the thermal lattice in
+ * kernels of their own, the fluid a step ahead; 1 = one block per row for both, its thermal input staged in shared
+ * memory by bulk copies while the fluid lattice runs (row lengths up to 320; longer ones run variant 0). A lattice
+ * starts with block 64 and the variant its size, storage and mask suggest. Variant 1 waits for its copies with a bounded wait; if a wait ever gives up, the call that sees it
  * (xac_lattice_stats, xac_lattice_run) returns XAC_ETIMEOUT and the lattice refuses every further step, run, stats,
  * fields, scalars, validate and save-state call with XAC_ETIMEOUT until xac_lattice_init_fields or
  * xac_lattice_load_state rewrites its populations. Results do not depend on the shape (every cell runs the same

@@ -8,6 +8,7 @@
 #include <tuple>
 #include <type_traits>
 #include <mutex>
+#include <set>
 #include <utility>
 #include <vector>
 
@@ -67,6 +68,20 @@ __global__ void build_link_kernel(const uint8_t* __restrict__ type, const float*
   if (z == g.nz - 1) w |= kZHiBit;
   if (w & (kYLoBit | kYHiBit | kZLoBit | kZHiBit)) w |= kYZBit;
   link[c] = w;
+}
+
+// the split step's list of non-solid cells, by slot
+__global__ void build_cells_kernel(const uint32_t* __restrict__ link, const uint2* __restrict__ ftab,
+                                   uint2* __restrict__ cells, Geom g) {
+  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (c >= g.ncell) return;
+  const uint32_t lw = link[c];
+  if (link_type(lw) == kSolid) return;
+  const uint32_t row = (uint32_t)(c / g.nx), x = (uint32_t)(c - (long long)row * g.nx);
+  const uint32_t t0 = ftab_index(g, row, x);
+  const uint2 e = ftab[t0];
+  cells[e.y + (uint32_t)__popc(e.x & ((1u << (x & 31u)) - 1u))] =
+      make_uint2((lw & ((1u << kCellXShift) - 1u)) | ((x & 31u) << kCellXShift), t0);
 }
 
 // ref-layout fields (any may be null = cold-start constant) -> internal rho, ux, uy, uz, T
@@ -150,11 +165,11 @@ __global__ void export_fields_kernel(const float* __restrict__ rho, const float*
 
 __global__ void set_scalar_kernel(float* dst, float v) { *dst = v; }
 
-// Memory-pattern probe of the fused step (SP / SQ: unsigned words of the fluid / thermal storage size): the
-// threads, the link-word and table reads, the population addresses (fluid pulls of the non-solid cells with the
-// bounce-back reads their link bits select, thermal pulls from the neighbours) and the whole-sector fills of the
-// thermal padding lanes that coupled_step_kernel has, with no arithmetic: every value read is stored unchanged at
-// the cell's own position of the other buffer. Its time is the floor the step's memory access pattern sets. (At the domain faces the thermal
+// Memory-pattern probe of a step (SP / SQ: unsigned words of the fluid / thermal storage size): both lattices in one
+// pass, one thread per row position, with the link-word and table reads, the population addresses (fluid pulls of the
+// non-solid cells with the bounce-back reads their link bits select, thermal pulls from the neighbours) and the
+// whole-sector fills of the thermal padding lanes, and no arithmetic: every value read is stored unchanged at the
+// cell's own position of the other buffer. Its time is what that access pattern takes. (At the domain faces the thermal
 // rules read the cell's own row instead of a neighbour: the probe pulls there too, which reads padding or guard
 // values.)
 template <typename SP, typename SQ, int kT>
@@ -176,7 +191,7 @@ __global__ void __launch_bounds__(256) pattern_copy_kernel(const SP* __restrict_
   const uint32_t e0 = pop_base(r, x, g, RL);
   if (fluid) {
     const FluidAt<SP> P = fluid_at(Pin, r, x, g, ftab);
-#define XAC_PC_P(I) Pout[P.k + (I) * P.ns] = ((lw >> (I)) & 1u) ? __ldg(P.own(opp_of(I))) : __ldg(P.template pull<I>());
+#define XAC_PC_P(I) Pout[P.own_index(I)] = ((lw >> (I)) & 1u) ? __ldg(P.own(opp_of(I))) : __ldg(P.template pull<I>());
     XAC_FOR19(XAC_PC_P)
 #undef XAC_PC_P
   }
@@ -297,6 +312,9 @@ static __global__ void run_decision_kernel(const double* __restrict__ st, RunCtl
 }
 
 // ---------------------------------------------------------------- the lattice object
+constexpr int kStatusSlot = 40;  // double of red_out / host_out that holds the status word
+static_assert(kStatusSlot >= kNStats && kStatusSlot >= kNMetrics && kStatusSlot >= kNValidate, "past every reduction");
+
 struct LatticeImpl {
   Geom g{};
   int precision = XAC_FP32;
@@ -306,9 +324,20 @@ struct LatticeImpl {
   float tau_th_f = 0.5f, tau_th_s = 0.5f;
   float relax[5] = {1.0f, 1.0f, 1.0f, 0.5f, 0.5f};  // omega_f, omega_tf, omega_ts, srcf_f, srcf_s (device-computed)
   float u_in_host = 0.0f;
-  int tune_block = 128;  // threads per block of the step kernel
-  int tune_variant = 0;  // 0: one thread per row position; 1: thermal rows staged in shared memory
-  unsigned* status = nullptr;  // device word set by a step kernel whose bounded wait ran out
+  int tune_block = 64;   // threads per block of the split step's kernels (128: +1 to +4%, 256: +8 to +12%)
+  int tune_variant = 0;  // 0: split step, the two lattices in kernels of their own; 1: thermal rows staged in shared memory
+  // The launch shape a lattice starts with. The staged step is one launch where the split step takes two, and wins where
+  // launches decide: at 98k row positions 5.7 against 6.6 us in FP32 and 5.9 against 6.8 in FP16; at 197k it is 9.5 against
+  // 9.0 and 10.0 against 9.2, at 655k 27.6 against 27.1 and 26.0 against 20.5. (Its one-warp blocks at row length 32 pay
+  // off in 16 bits only: 30x20x12 4.9 against 4.3 us in FP32, 5.2 against 5.8 in FP16.) In FP32, where memory decides, it
+  // also wins where rows are all fluid or all solid and the split step has no idle lanes to save: straight channels
+  // 148x128x32 26.8 against 27.5 us, 301x203x61 148 against 159; at 60% full warps (pins) 24.3 against 23.2.
+  void default_tune(double full_lanes) {
+    const bool small = (long long)g.rows * g.pitch <= 131072;
+    const bool staged = small ? g.pitch >= 64 || precision != XAC_FP32 : precision == XAC_FP32 && full_lanes >= 0.8;
+    tune_variant = staged && g.pitch <= kMaxStagedRow ? 1 : 0;
+  }
+  unsigned* status = nullptr;  // device word set by a step kernel whose bounded wait ran out (in red_out's tail)
   // set once the status word was seen non-zero: a staged step gave up on its copies, so the thermal populations it
   // wrote are not the step's; the lattice refuses work until init_fields / load_state rewrites its populations
   bool failed = false;
@@ -325,6 +354,11 @@ struct LatticeImpl {
   uint32_t* link = nullptr;
   uint2* ftab = nullptr;  // non-solid cell table of the fluid populations
   uint32_t nonsolid = 0;  // non-solid cells (the fluid populations' slots in use)
+  uint2* cells = nullptr;    // the split step's non-solid cells, by slot
+  uint32_t* ends = nullptr;  // slots of the inlet and outlet cells
+  uint32_t nends = 0;
+  static constexpr int kUSets = 2;  // three sets measured the same
+  float* u_step = nullptr;  // [kUSets][3][ncell]: u by slot, from the fluid's step to the thermal lattice's
   float* qsrc = nullptr;
   float* u_in = nullptr;
   float *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr, *T = nullptr;
@@ -345,7 +379,15 @@ struct LatticeImpl {
   }
   long long macro_step = 0;   // rho/u arrays hold the fields of this step
   long long T_step = 0;       // T array holds the field of this step
-  cudaStream_t capture = nullptr;
+  cudaStream_t capture = nullptr, fluid_branch = nullptr;
+  std::vector<cudaEvent_t> events;  // order of the captured branches
+  cudaError_t capture_streams() {
+    cudaError_t e = cudaSuccess;
+    if (!capture) e = cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !fluid_branch) e = cudaStreamCreateWithFlags(&fluid_branch, cudaStreamNonBlocking);
+    return e;
+  }
+  std::set<std::pair<int, int>> called;                   // (n, parity) of launch_graph calls so far
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (n, parity) -> n steps with macro output at the end
   std::map<std::pair<int, int>, cudaGraphExec_t> run_graphs;  // (stats_every, parity) -> device-resident run loop
   RunCtl* run_ctl = nullptr;       // device
@@ -381,8 +423,10 @@ struct LatticeImpl {
     cudaFree(type);
     cudaFree(link);
     cudaFree(ftab);
+    cudaFree(cells);
+    cudaFree(ends);
+    cudaFree(u_step);
     cudaFree(qsrc);
-    cudaFree(status);
     cudaFree(u_in);
     cudaFree(rho);
     cudaFree(ux);
@@ -393,25 +437,120 @@ struct LatticeImpl {
     cudaFree(red_out);
     if (host_out) cudaFreeHost(host_out);
     if (capture) cudaStreamDestroy(capture);
+    if (fluid_branch) cudaStreamDestroy(fluid_branch);
+    for (cudaEvent_t ev : events) cudaEventDestroy(ev);
   }
 
-  template <int kPrec>
-  int launch_step(cudaStream_t s, bool macro, bool own) {
-    const StepParams p = params();
-    StepLaunch a{P[cur], P[cur ^ 1], Qb[cur], Qb[cur ^ 1], link, qsrc, u_in, rho, ux, uy, uz, T, p, tune_block,
-                 tune_variant, macro, own, s};
-    launch_coupled_step<typename Storage<kPrec>::P, typename Storage<kPrec>::Q>(a);
-    cur ^= 1;
-    return XAC_OK;
-  }
+  bool staged() const { return tune_variant == 1 && g.pitch <= kMaxStagedRow; }
 
-  int launch_step_any(cudaStream_t s, bool macro, bool own) {
+  void launch_staged(cudaStream_t s, bool macro, bool own) {
+    const StepLaunch a{P[cur], P[cur ^ 1], Qb[cur], Qb[cur ^ 1], link, qsrc, u_in, rho, ux, uy, uz, T, params(),
+                       macro, own, s};
     switch (precision) {
-      case XAC_FP16: return launch_step<XAC_FP16>(s, macro, own);
-      case XAC_BF16: return launch_step<XAC_BF16>(s, macro, own);
-      case XAC_FP32_T16: return launch_step<XAC_FP32_T16>(s, macro, own);
-      default: return launch_step<XAC_FP32>(s, macro, own);
+      case XAC_FP16: launch_staged_step<__half, __half>(a); break;
+      case XAC_BF16: launch_staged_step<__nv_bfloat16, __half>(a); break;
+      case XAC_FP32_T16: launch_staged_step<float, __half>(a); break;
+      default: launch_staged_step<float, float>(a);
     }
+    cur ^= 1;
+  }
+
+  // One launch of the split step in a run of n: the fluid lattice's step f (1..n, 0: none) and the thermal lattice's step
+  // t (0: none). c0 is the buffer parity before the run. The last step also writes rho and u to the field arrays.
+  void launch_split(cudaStream_t s, int n, int c0, int f, int t, bool own) {
+    SplitArgs a{};
+    const int cf = (c0 + f + 1) & 1, ct = (c0 + t + 1) & 1;  // parity of the buffers step f / t reads
+    float* const field[3] = {ux, uy, uz};
+    auto uset = [&](int back, int k) { return u_step + ((size_t)(back % kUSets) * 3 + k) * g.ncell; };
+    a.p = params();
+    a.link = link;
+    a.qsrc = qsrc;
+    a.u_in = u_in;
+    a.cells = cells;
+    a.ends = ends;
+    a.T0 = T;
+    a.nfluid = nonsolid;
+    a.nends = nends;
+    const unsigned B = (unsigned)tune_block;
+    if (f > 0) {
+      a.Pin = P[cf];
+      a.Pout = P[cf ^ 1];
+      a.fblocks = (nonsolid + B - 1) / B;
+      a.eblocks = (nends + B - 1) / B;
+      a.frev = (uint32_t)cf;
+      if (f == n) {
+        a.field[0] = rho;
+        for (int k = 0; k < 3; ++k) a.field[1 + k] = field[k];
+      }
+      for (int k = 0; k < 3; ++k) a.uo[k] = uset(n - f, k);
+    }
+    if (t > 0) {
+      a.Qin = Qb[ct];
+      a.Qout = Qb[ct ^ 1];
+      a.tblocks = (unsigned)(((long long)g.rows * g.pitch + B - 1) / B);
+      a.trev = (uint32_t)ct;
+      a.own = own ? 1 : 0;
+      for (int k = 0; k < 3; ++k) a.ui[k] = uset(n - t, k);
+      if (t == n) {
+        a.solid[0] = rho;
+        for (int k = 0; k < 3; ++k) a.solid[1 + k] = field[k];
+      }
+    }
+    const bool plain = !own && !a.field[0] && !a.solid[0];
+    if (a.fblocks + a.eblocks > 0) switch (precision) {  // none in an all-solid lattice
+        case XAC_FP16: launch_split_fluid<__half>(a, tune_block, plain, s); break;
+        case XAC_BF16: launch_split_fluid<__nv_bfloat16>(a, tune_block, plain, s); break;
+        default: launch_split_fluid<float>(a, tune_block, plain, s);
+      }
+    if (t > 0) {
+      if (precision == XAC_FP32) launch_split_thermal<float>(a, tune_block, plain, s);
+      else launch_split_thermal<__half>(a, tune_block, plain, s);
+    }
+  }
+
+  // n steps, the last one writing rho/u; own: the first one reads the initial thermal populations unstreamed
+  void launch_steps(cudaStream_t s, int n, bool own) {
+    if (staged()) {
+      for (int k = 0; k < n; ++k) launch_staged(s, k == n - 1, own && k == 0);
+      return;
+    }
+    for (int k = 1; k <= n; ++k) {
+      launch_split(s, n, cur, k, 0, false);
+      launch_split(s, n, cur, 0, k, own && k == 1);
+    }
+    if (n & 1) cur ^= 1;
+  }
+
+  // The same with the two lattices on two branches, captured or not: thermal step k waits for fluid step k, fluid step k
+  // for thermal step k - kUSets (whose velocity it overwrites). The branches join on st.
+  cudaError_t branch_steps(cudaStream_t st, int n) {
+    if (staged()) {
+      launch_steps(st, n, false);
+      return cudaSuccess;
+    }
+    // an event may be recorded again once its waits are issued: a ring of thermal ones, one fluid one
+    cudaError_t e = cudaSuccess;
+    auto ck = [&](cudaError_t r) {
+      if (e == cudaSuccess) e = r;
+    };
+    while (events.size() < kUSets + 1) {
+      cudaEvent_t ev = nullptr;
+      if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
+      events.push_back(ev);
+    }
+    const cudaEvent_t fluid_done = events[kUSets];
+    ck(cudaEventRecord(fluid_done, st));
+    ck(cudaStreamWaitEvent(fluid_branch, fluid_done, 0));
+    for (int k = 1; k <= n; ++k) {
+      if (k > kUSets) ck(cudaStreamWaitEvent(fluid_branch, events[k % kUSets], 0));
+      launch_split(fluid_branch, n, cur, k, 0, false);
+      ck(cudaEventRecord(fluid_done, fluid_branch));
+      ck(cudaStreamWaitEvent(st, fluid_done, 0));
+      launch_split(st, n, cur, 0, k, false);
+      ck(cudaEventRecord(events[k % kUSets], st));
+    }
+    if (n & 1) cur ^= 1;
+    return e;
   }
 
   // T of the current state into the T field (the thermal populations' storage type follows the precision mode)
@@ -424,26 +563,27 @@ struct LatticeImpl {
       thermal_finalize_kernel<__half><<<grid, kBlock, 0, s>>>((const __half*)Qb[cur], link, T, p);
   }
 
-  // n plain steps (no own step), the last one writing rho/u
-  int launch_plain(cudaStream_t s, int n) {
-    for (int k = 0; k < n; ++k) {
-      int r = launch_step_any(s, k == n - 1, false);
-      if (r != XAC_OK) return r;
-    }
-    return XAC_OK;
-  }
-
-  // n >= 8 plain steps from the cached graph of n steps for the current buffer parity (captured on first use)
+  // n >= 8 plain steps. The first call of a length launches them one by one, later ones from a graph: capturing and
+  // instantiating 100 steps costs 0.5-0.9 ms, which a lattice that makes the call once would pay for nothing (the GPU is
+  // no slower: launching a step takes less than running it).
   int launch_graph(cudaStream_t s, int n) {
+    XAC_CUDA(capture_streams());
     auto key = std::make_pair(n, cur);
     auto it = graphs.find(key);
+    if (it == graphs.end() && called.insert(key).second) {
+      XAC_CUDA(branch_steps(s, n));
+      return XAC_OK;
+    }
     if (it == graphs.end()) {
-      if (!capture) XAC_CUDA(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
       const int saved = cur;
       cudaGraph_t graph = nullptr;
       XAC_CUDA(cudaStreamBeginCapture(capture, cudaStreamCaptureModeThreadLocal));
-      launch_plain(capture, n);
+      const cudaError_t ce = branch_steps(capture, n);
       cudaError_t e = cudaStreamEndCapture(capture, &graph);
+      if (e == cudaSuccess && ce != cudaSuccess) {
+        cudaGraphDestroy(graph);
+        e = ce;
+      }
       cur = saved;
       if (e != cudaSuccess) return cuda_status(e, "cudaStreamEndCapture");
       cudaGraphExec_t exec = nullptr;
@@ -457,13 +597,13 @@ struct LatticeImpl {
     return XAC_OK;
   }
 
-  // Long runs go as graphs of at most kGraphSteps steps (an even count, so the same graph serves every chunk);
-  // each chunk's last step also writes rho/u, which changes no population.
+  // Long runs go as graphs of at most kGraphSteps steps (an even count, so the same graph serves every chunk); each
+  // chunk's last step also writes rho/u, which changes no population.
   static constexpr int kGraphSteps = 512;
   int steps(int n, cudaStream_t s) {
     if (n <= 0) return XAC_OK;
     if (own_pending) {
-      launch_step_any(s, n == 1, true);
+      launch_steps(s, 1, true);
       own_pending = false;
       step += 1;
       --n;
@@ -479,7 +619,7 @@ struct LatticeImpl {
         int r = launch_graph(s, n);
         if (r != XAC_OK) return r;
       } else {
-        launch_plain(s, n);
+        launch_steps(s, n, false);
       }
       step += total;
       XAC_CUDA(cudaGetLastError());
@@ -498,7 +638,7 @@ struct LatticeImpl {
       *out = it->second;
       return XAC_OK;
     }
-    if (!capture) XAC_CUDA(cudaStreamCreateWithFlags(&capture, cudaStreamNonBlocking));
+    XAC_CUDA(capture_streams());
     if (!run_ctl) XAC_CUDA(cudaMalloc(&run_ctl, sizeof(RunCtl)));
     if (!run_ctl_host) XAC_CUDA(cudaMallocHost(&run_ctl_host, sizeof(RunCtl)));
     cudaGraph_t graph = nullptr;
@@ -520,7 +660,7 @@ struct LatticeImpl {
       cudaGraphDestroy(graph);
       return cuda_status(e, "run loop graph");
     }
-    launch_plain(capture, every);
+    const cudaError_t ce = branch_steps(capture, every);
     launch_finalize_T(capture);
     const auto spec = stats_spec();
     const int ntiles = (int)stats_tiles(g.ncell);
@@ -529,6 +669,7 @@ struct LatticeImpl {
     run_decision_kernel<<<1, 1, 0, capture>>>(red_out, run_ctl, u_in, h);
     cudaGraph_t body = nullptr;
     e = cudaStreamEndCapture(capture, &body);
+    if (e == cudaSuccess) e = ce;
     cur = saved;
     cudaGraphExec_t exec = nullptr;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
@@ -569,13 +710,14 @@ struct LatticeImpl {
 
 // ---------------------------------------------------------------- shared reduction drivers
 // rows must hold stats_tiles(cells) * kNStats doubles
-int run_stats(const FieldView& v, double* rows, double* dev_out, double* host_out, cudaStream_t s) {
+int run_stats(const FieldView& v, double* rows, double* dev_out, double* host_out, cudaStream_t s,
+              int copied = kNStats) {
   const auto spec = stats_spec();
   const int ntiles = (int)stats_tiles((long long)v.nx * v.ny * v.nz);
   stats_partials_kernel<<<ntiles, kStatsBlock, 0, s>>>(v, spec, rows);
   combine_rows_kernel<kNStats><<<1, 32 * kNStats, 0, s>>>(rows, ntiles, spec, dev_out);
   XAC_CUDA(cudaGetLastError());
-  XAC_CUDA(cudaMemcpyAsync(host_out, dev_out, kNStats * sizeof(double), cudaMemcpyDeviceToHost, s));
+  XAC_CUDA(cudaMemcpyAsync(host_out, dev_out, copied * sizeof(double), cudaMemcpyDeviceToHost, s));
   XAC_CUDA(cudaStreamSynchronize(s));
   return XAC_OK;
 }
@@ -663,8 +805,8 @@ namespace {
 // Normalised heat source times power, internal layout; simulation.py:77-86 and thermal_engine3d.py:116-117.
 // Table of the fluid populations' non-solid cells (FluidAt): per 32-cell word of each row its non-solid mask and
 // the number of non-solid cells before it, with ny + 1 empty rows before and after the grid. Sets g.nt, g.ns and
-// g.np. type is in cell order c = (z*ny + y)*nx + x.
-std::vector<uint2> fluid_table(const uint8_t* type, Geom& g, uint32_t* nonsolid) {
+// g.np; ends receives the slots of the inlet and outlet cells. type is in cell order c = (z*ny + y)*nx + x.
+std::vector<uint2> fluid_table(const uint8_t* type, Geom& g, uint32_t* nonsolid, std::vector<uint32_t>* ends) {
   g.nt = g.pitch / 32;
   const long long guard_rows = g.ny + 1;
   std::vector<uint2> tab((size_t)((g.rows + 2 * guard_rows) * g.nt), make_uint2(0u, 0u));
@@ -674,7 +816,10 @@ std::vector<uint2> fluid_table(const uint8_t* type, Geom& g, uint32_t* nonsolid)
       uint32_t m = 0;
       for (int b = 0; b < 32; ++b) {
         const int x = 32 * w + b;
-        if (x < g.nx && type[r * g.nx + x] != kSolid) m |= 1u << b;
+        if (x < g.nx && type[r * g.nx + x] != kSolid) {
+          if (type[r * g.nx + x] != kFluid) ends->push_back(k + (uint32_t)__builtin_popcount(m));
+          m |= 1u << b;
+        }
       }
       tab[(size_t)((r + guard_rows) * g.nt + w)] = make_uint2(m, k);
       k += (uint32_t)__builtin_popcount(m);
@@ -685,6 +830,7 @@ std::vector<uint2> fluid_table(const uint8_t* type, Geom& g, uint32_t* nonsolid)
   g.ns = ((long long)k + 31) / 32 * 32;
   if (g.ns == 0) g.ns = 32;
   g.np = (long long)kQ * g.ns;
+  for (int i = 0; i < kQ; ++i) g.run[i] = (uint32_t)((long long)i * g.ns);
   return tab;
 }
 
@@ -737,6 +883,10 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   L.g.rows = ny * nz;
   L.g.guard = (long long)(ny + 2) * kQ * L.g.pitch;
   L.g.N = (long long)L.g.rows * kQ * L.g.pitch + 2 * L.g.guard;
+  for (int i = 0; i < kQ; ++i) {
+    L.g.own_off[i] = (uint32_t)(i * L.g.pitch);
+    L.g.pull_off[i] = (uint32_t)((i - ey_of(i) * kQ) * L.g.pitch - ex_of(i));
+  }
   L.precision = d->precision;
   L.p_elem = (d->precision == XAC_FP32 || d->precision == XAC_FP32_T16) ? 4 : 2;
   L.q_elem = d->precision == XAC_FP32 ? 4 : 2;
@@ -764,7 +914,14 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
         type[((size_t)z * ny + y) * nx + x] = (uint8_t)m;
       }
   std::vector<float> q = host_qsrc(d);
-  const std::vector<uint2> ftab = fluid_table(type.data(), L.g, &L.nonsolid);
+  std::vector<uint32_t> ends;
+  const std::vector<uint2> ftab = fluid_table(type.data(), L.g, &L.nonsolid, &ends);
+  L.nends = (uint32_t)ends.size();
+  {
+    long long words = 0;  // warps of the one-pass step that hold a non-solid cell
+    for (const uint2& e : ftab) words += e.x != 0u;
+    L.default_tune(words ? (double)L.nonsolid / (32.0 * words) : 0.0);
+  }
   const size_t p_bytes = (size_t)L.g.np * L.p_elem, q_bytes = (size_t)L.g.N * L.q_elem;
   for (int b = 0; b < 2; ++b) {
     XAC_CUDA(cudaMalloc(&L.P[b], p_bytes));
@@ -774,10 +931,11 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   if ((r = dmalloc(&L.type, n, "alloc type")) != XAC_OK) return r;
   if ((r = dmalloc(&L.link, n, "alloc link")) != XAC_OK) return r;
   if ((r = dmalloc(&L.ftab, ftab.size(), "alloc fluid table")) != XAC_OK) return r;
+  if ((r = dmalloc(&L.cells, n, "alloc cell list")) != XAC_OK) return r;
+  if ((r = dmalloc(&L.ends, ends.size(), "alloc inlet and outlet list")) != XAC_OK) return r;
+  if ((r = dmalloc(&L.u_step, 3 * LatticeImpl::kUSets * (size_t)n, "alloc velocity")) != XAC_OK) return r;
   if ((r = dmalloc(&L.qsrc, n, "alloc qsrc")) != XAC_OK) return r;
   if ((r = dmalloc(&L.u_in, 1, "alloc u_in")) != XAC_OK) return r;
-  if ((r = dmalloc(&L.status, 1, "alloc status")) != XAC_OK) return r;
-  XAC_CUDA(cudaMemsetAsync(L.status, 0, sizeof(unsigned), s));
   for (float** f : {&L.rho, &L.ux, &L.uy, &L.uz, &L.T})
     if ((r = dmalloc(f, n, "alloc fields")) != XAC_OK) return r;
   L.red_blocks = reduction_blocks(n);
@@ -786,6 +944,8 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
     if ((r = dmalloc(&L.rows, metric_rows > stat_rows ? metric_rows : stat_rows, "alloc rows")) != XAC_OK) return r;
   }
   if ((r = dmalloc(&L.red_out, 64, "alloc red_out")) != XAC_OK) return r;
+  L.status = reinterpret_cast<unsigned*>(L.red_out + kStatusSlot);
+  XAC_CUDA(cudaMemsetAsync(L.red_out + kStatusSlot, 0, sizeof(double), s));
   XAC_CUDA(cudaMallocHost(&L.host_out, 64 * sizeof(double)));
   // guards, row padding and the unused fluid slots are never used as values; keep them defined
   for (int b = 0; b < 2; ++b) {
@@ -795,10 +955,13 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   XAC_CUDA(cudaMemcpyAsync(L.type, type.data(), n, cudaMemcpyHostToDevice, s));
   XAC_CUDA(cudaMemcpyAsync(L.ftab, ftab.data(), ftab.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
   XAC_CUDA(cudaMemcpyAsync(L.qsrc, q.data(), n * sizeof(float), cudaMemcpyHostToDevice, s));
+  if (!ends.empty())
+    XAC_CUDA(cudaMemcpyAsync(L.ends, ends.data(), ends.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   set_scalar_kernel<<<1, 1, 0, s>>>(L.u_in, L.u_in_host);
   relaxation_factors_kernel<<<1, 1, 0, s>>>((float)L.tau_fluid, L.tau_th_f, L.tau_th_s, (float*)L.red_out);
   XAC_CUDA(cudaMemcpyAsync(L.relax, L.red_out, sizeof(L.relax), cudaMemcpyDeviceToHost, s));
   build_link_kernel<<<grid_for(n, kBlock), kBlock, 0, s>>>(L.type, L.qsrc, L.link, L.g);
+  build_cells_kernel<<<grid_for(n, kBlock), kBlock, 0, s>>>(L.link, L.ftab, L.cells, L.g);
   XAC_CUDA(cudaGetLastError());
   // host vectors go out of scope: make the copies complete first
   XAC_CUDA(cudaStreamSynchronize(s));
@@ -907,13 +1070,12 @@ int xac_lattice_stats(xac_lattice* lat, double* out_host, void* stream) {
   cudaStream_t s = as_stream(stream);
   int r = L.finalize_T(s);
   if (r != XAC_OK) return r;
-  r = run_stats(L.view(), L.rows, L.red_out, L.host_out, s);
+  r = run_stats(L.view(), L.rows, L.red_out, L.host_out, s, L.staged() ? kStatusSlot + 1 : kNStats);
   if (r != XAC_OK) return r;
   std::memcpy(out_host, L.host_out, kNStats * sizeof(double));
-  if (L.tune_variant == 1) {  // the staged kernel's bounded wait reports here
+  if (L.staged()) {  // the staged kernel's bounded wait reports here
     unsigned st = 0;
-    XAC_CUDA(cudaMemcpyAsync(&st, L.status, sizeof(st), cudaMemcpyDeviceToHost, s));
-    XAC_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(&st, L.host_out + kStatusSlot, sizeof(st));
     if (st) {
       L.failed = true;
       set_error("xac_lattice_stats: a staged step kernel gave up waiting for its copies (status %u); the lattice "
@@ -1287,7 +1449,7 @@ int xac_lattice_run(xac_lattice* lat, const xac_run_opts* o, xac_run_result* res
       dT = c.dT;
       dQ = c.dQ;
       std::memcpy(res->last_stats, c.last, sizeof(c.last));
-      if (L.tune_variant == 1) {  // the staged kernel's bounded wait reports here
+      if (L.staged()) {  // the staged kernel's bounded wait reports here
         unsigned stw = 0;
         XAC_CUDA(cudaMemcpy(&stw, L.status, sizeof(stw), cudaMemcpyDeviceToHost));
         if (stw) {
@@ -1884,17 +2046,21 @@ int xac_lattice_footprint(const xac_desc* d, unsigned long long* bytes) {
   const long long pitch = (d->nx + 31) / 32 * 32;
   const long long N = ((long long)d->ny * d->nz + 2LL * (d->ny + 2)) * kQ * pitch;
   // fluid populations of the non-solid cells (all cells when no mask is given)
-  long long nonsolid = n;
+  long long nonsolid = n, ends = 0;
   if (d->mask) {
     nonsolid = 0;
-    for (long long c = 0; c < n; ++c) nonsolid += d->mask[c] != kSolid;
+    for (long long c = 0; c < n; ++c) {
+      nonsolid += d->mask[c] != kSolid;
+      ends += d->mask[c] == kInlet || d->mask[c] == kOutlet;
+    }
   }
   const long long NP = kQ * ((nonsolid + 31) / 32 * 32 + (nonsolid == 0 ? 32 : 0));
   const long long ftab = ((long long)d->ny * d->nz + 2LL * (d->ny + 1)) * (pitch / 32) * 8;
   const long long p_elem = (d->precision == XAC_FP32 || d->precision == XAC_FP32_T16) ? 4 : 2;
   const long long q_elem = d->precision == XAC_FP32 ? 4 : 2;
   const long long metric_rows = (long long)reduction_blocks(n) * kNMetrics, stat_rows = stats_tiles(n) * kNStats;
-  *bytes = (unsigned long long)(2 * NP * p_elem + 2 * N * q_elem + ftab + n * (1 + 4 + 4 + 5 * 4) +
+  *bytes = (unsigned long long)(2 * NP * p_elem + 2 * N * q_elem + ftab + 4 * ends +
+                                n * (1 + 4 + 4 + 8 + 5 * 4 + 6 * 4) +
                                 8 * (metric_rows > stat_rows ? metric_rows : stat_rows) + 64 * 8 + 64);
   return XAC_OK;
 }

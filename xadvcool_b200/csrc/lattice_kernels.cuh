@@ -68,6 +68,10 @@ struct Geom {
   int nt;           // 32-cell words of a row: pitch / 32
   long long ns;     // slots of a fluid population run: the non-solid cells, rounded up to a multiple of 32
   long long np;     // elements of one fluid population array: 19*ns
+  uint32_t run[kQ];  // start of each direction's run: i*ns
+  // thermal populations: own value of direction i (i*pitch); its source ((i - e_y*19)*pitch - e_x) from the row one z-slab
+  // against e_z
+  uint32_t own_off[kQ], pull_off[kQ];
 };
 
 // row length, a compile-time constant when kT > 0
@@ -178,17 +182,17 @@ struct Rows {
   }
 };
 // Runtime row length: one base pointer and 32-bit element indices (every index of a population array fits in 31
-// bits), so an address is formed right before its load instead of 19 64-bit pointers living at once.
+// bits); the offsets are kernel parameters, constant operands of the index additions.
 template <typename S>
 struct Rows<S, 0> {
   const S* base;
   uint32_t c, zm, zp;
-  int RL;
-  __device__ __forceinline__ const S* own(int i) const { return base + (c + (uint32_t)(i * RL)); }
+  const Geom* g;
+  __device__ __forceinline__ const S* own(int i) const { return base + (c + g->own_off[i]); }
   template <int I>
   __device__ __forceinline__ const S* pull() const {
     const uint32_t b = ez_of(I) > 0 ? zm : (ez_of(I) < 0 ? zp : c);
-    return base + (b + (uint32_t)((I - ey_of(I) * kQ) * RL - ex_of(I)));
+    return base + (b + g->pull_off[I]);
   }
 };
 template <int kT, typename S>
@@ -198,7 +202,7 @@ __device__ __forceinline__ Rows<S, kT> rows_at(const S* base, uint32_t e0, const
     return {base + e0, base + e0 - slab, base + e0 + slab, pitch};
   } else {
     const uint32_t slab = (uint32_t)g.ny * kQ * (uint32_t)pitch;
-    return {base, e0, e0 - slab, e0 + slab, pitch};
+    return {base, e0, e0 - slab, e0 + slab, &g};
   }
 }
 
@@ -223,11 +227,13 @@ __host__ __device__ constexpr int fluid_row_ez(int j) { return j == 2 || j == 4 
 template <typename S>
 struct FluidAt {
   const S* base;
-  uint32_t ns, k, nb;
+  const uint32_t* run;  // run[i] = i*ns (kernel parameters: a constant operand of the index additions)
+  uint32_t k, nb;
   uint32_t rk[8];
-  __device__ __forceinline__ const S* own(int i) const { return base + ((uint32_t)i * ns + k); }
+  __device__ __forceinline__ uint32_t own_index(int i) const { return k + run[i]; }
+  __device__ __forceinline__ const S* own(int i) const { return base + own_index(i); }
   template <int I>
-  __device__ __forceinline__ const S* pull() const {
+  __device__ __forceinline__ uint32_t pull_index() const {
     uint32_t s;
     if constexpr (ey_of(I) == 0 && ez_of(I) == 0) {
       s = k - (uint32_t)ex_of(I);
@@ -237,24 +243,26 @@ struct FluidAt {
       if constexpr (ex_of(I) == 1) s -= 1u;
       if constexpr (ex_of(I) == -1) s += (nb >> j) & 1u;
     }
-    return base + ((uint32_t)I * ns + s);
+    return s + run[I];
+  }
+  template <int I>
+  __device__ __forceinline__ const S* pull() const {
+    return base + pull_index<I>();
   }
 };
 // table entry of the word holding cell (row r, x)
 __host__ __device__ __forceinline__ uint32_t ftab_index(const Geom& g, uint32_t r, uint32_t x) {
   return (r + (uint32_t)g.ny + 1u) * (uint32_t)g.nt + (x >> 5);
 }
-// the view of cell (row r, x), which must be non-solid; the nine table loads are the same for a whole warp
+// the view of the non-solid cell in slot k, bit `bit` of table entry t0
 template <typename S>
-__device__ __forceinline__ FluidAt<S> fluid_at(const S* base, uint32_t r, uint32_t x, const Geom& g,
-                                               const uint2* __restrict__ ftab) {
+__device__ __forceinline__ FluidAt<S> fluid_at_entry(const S* base, uint32_t k, uint32_t t0, uint32_t bit, const Geom& g,
+                                                     const uint2* __restrict__ ftab) {
   FluidAt<S> a;
   a.base = base;
-  a.ns = (uint32_t)g.ns;
-  const uint32_t below = (1u << (x & 31u)) - 1u, bit = x & 31u;
-  const uint32_t t0 = ftab_index(g, r, x);
-  const uint2 e = __ldg(ftab + t0);
-  a.k = e.y + (uint32_t)__popc(e.x & below);
+  a.run = g.run;
+  a.k = k;
+  const uint32_t below = (1u << bit) - 1u;
   a.nb = 0u;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -265,7 +273,17 @@ __device__ __forceinline__ FluidAt<S> fluid_at(const S* base, uint32_t r, uint32
   }
   return a;
 }
+// the view of cell (row r, x), which must be non-solid; the nine table loads are the same for a whole warp
+template <typename S>
+__device__ __forceinline__ FluidAt<S> fluid_at(const S* base, uint32_t r, uint32_t x, const Geom& g,
+                                               const uint2* __restrict__ ftab) {
+  const uint32_t t0 = ftab_index(g, r, x), bit = x & 31u;
+  const uint2 e = __ldg(ftab + t0);
+  return fluid_at_entry(base, e.y + (uint32_t)__popc(e.x & ((1u << bit) - 1u)), t0, bit, g, ftab);
+}
 
+// the nine pairs of opposite directions
+#define XAC_PAIRS(M) M(1, 2) M(3, 4) M(5, 6) M(7, 8) M(9, 10) M(11, 12) M(13, 14) M(15, 16) M(17, 18)
 #define XAC_FOR19(M) M(0) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) M(16) M(17) M(18)
 
 // Lanes sharing one 32-byte DRAM sector of a thermal population row (rows start on 32-value boundaries).
@@ -281,16 +299,11 @@ __device__ __forceinline__ unsigned sector_group(int lane) {
 // Po its own slot in the output (direction i at +i*ns); Q is its row view of the input thermal populations and Qo
 // its own position in the output (direction i at +i*pitch).
 
-// fluid lattice of a non-solid cell: pull with the boundary rules, moments, BGK collision; returns u
-template <typename S, bool kMacro, int kLd, class Acc>
-__device__ __forceinline__ void fluid_cell(const uint32_t c, const Acc& P, S* __restrict__ Po,
-                                           const float* __restrict__ u_in_ptr, float* __restrict__ rho_o,
-                                           float* __restrict__ ux_o, float* __restrict__ uy_o,
-                                           float* __restrict__ uz_o, const StepParams& p, const uint32_t lw,
-                                           float& ux, float& uy, float& uz) {
-  const int type = link_type(lw);
-  float F[kQ];
-  if (type == kInlet) {
+// Populations streamed to an inlet or outlet cell
+template <typename S, int kLd, class Acc>
+__device__ __forceinline__ void fluid_gather_end(const Acc& P, const float* __restrict__ u_in_ptr, const StepParams& p,
+                                                 const uint32_t lw, float (&F)[kQ]) {
+  if (link_type(lw) == kInlet) {
     // src/fluid_engine3d.py:197-244: no pull; unknown populations from the known ones
     float k[kQ];
 #define XAC_LD_OWN(I) k[I] = Pop<S>::template ld<kLd>(P.own(I), w_of(I));
@@ -321,7 +334,7 @@ __device__ __forceinline__ void fluid_cell(const uint32_t c, const Acc& P, S* __
     F[16] = k[16];
     F[17] = k[17];
     F[18] = k[18];
-  } else if (type == kOutlet) {
+  } else {
     // src/fluid_engine3d.py:247-259: copy post-collision (x-1) and rescale to rho_outlet. The x-1 cell is the
     // previous non-solid cell when it is not solid (link bit 1: the source of direction 1 is x-1), and holds the
     // rest equilibrium w_i when it is.
@@ -338,13 +351,28 @@ sum += F[I];
 #pragma unroll
       for (int i = 0; i < kQ; ++i) F[i] *= sc;
     }
-  } else {
-    // src/fluid_engine3d.py:262-272: pull, halfway bounce-back on out-of-domain or solid sources
-#define XAC_LD_PULL(I)                                                                                      \
-F[I] = ((lw >> I) & 1u) ? Pop<S>::template ld<kLd>(P.own(opp_of(I)), w_of(I)) : Pop<S>::template ld<kLd>(P.template pull<I>(), w_of(I));
-    XAC_FOR19(XAC_LD_PULL)
-#undef XAC_LD_PULL
   }
+}
+
+// Populations streamed to a fluid cell: pull, halfway bounce-back on out-of-domain or solid sources
+// (src/fluid_engine3d.py:262-272). The element is selected before the load: one address and one load a direction.
+template <typename S, int kLd, class Acc>
+__device__ __forceinline__ void fluid_gather(const Acc& P, const uint32_t lw, float (&F)[kQ]) {
+#define XAC_LD_PULL(I)                                                                                   \
+  {                                                                                                      \
+    const uint32_t e = ((lw >> (I)) & 1u) ? P.own_index(opp_of(I)) : P.template pull_index<I>();         \
+    F[I] = Pop<S>::template ld<kLd>(P.base + e, w_of(I));                                                \
+  }
+  XAC_FOR19(XAC_LD_PULL)
+#undef XAC_LD_PULL
+}
+
+// Moments and BGK collision of a non-solid cell; returns rho and u
+template <typename S, bool kMacro, class Acc>
+__device__ __forceinline__ void fluid_collide(const uint32_t c, const Acc& P, S* __restrict__ Po,
+                                              float* __restrict__ rho_o, float* __restrict__ ux_o,
+                                              float* __restrict__ uy_o, float* __restrict__ uz_o, const StepParams& p,
+                                              const float (&F)[kQ], float& rho, float& ux, float& uy, float& uz) {
   // src/fluid_engine3d.py:85-113 moments, reference summation order
   float r = 0.0f, mx = 0.0f, my = 0.0f, mz = 0.0f;
 #pragma unroll
@@ -365,16 +393,34 @@ F[I] = ((lw >> I) & 1u) ? Pop<S>::template ld<kLd>(P.own(opp_of(I)), w_of(I)) : 
     uy_o[c] = uy;
     uz_o[c] = uz;
   }
+  rho = r;
   // src/fluid_engine3d.py:157-173 BGK with the equilibrium in registers
   const float omega = p.omega_f;
   const float usq15 = 1.5f * ((ux * ux + uy * uy) + uz * uz);
-#define XAC_COLLIDE(I)                                                            \
-{                                                                               \
-  const float fe = feq_term(w_of(I) * r, edotu<I>(ux, uy, uz), usq15);         \
-  Pop<S>::st(Po + (I) * P.ns, F[I] - omega * (F[I] - fe), w_of(I));           \
-}
-  XAC_FOR19(XAC_COLLIDE)
+#define XAC_COLLIDE(I, J)                                                          \
+  {                                                                                \
+    float fi, fj;                                                                  \
+    feq_pair(w_of(I) * r, edotu<I>(ux, uy, uz), usq15, fi, fj);                    \
+    Pop<S>::st(Po + P.own_index(I), F[I] - omega * (F[I] - fi), w_of(I));          \
+    Pop<S>::st(Po + P.own_index(J), F[J] - omega * (F[J] - fj), w_of(J));          \
+  }
+  const float f0 = (w_of(0) * r) * (1.0f - usq15);
+  Pop<S>::st(Po + P.own_index(0), F[0] - omega * (F[0] - f0), w_of(0));
+  XAC_PAIRS(XAC_COLLIDE)
 #undef XAC_COLLIDE
+}
+
+// fluid lattice of a non-solid cell
+template <typename S, bool kMacro, int kLd, class Acc>
+__device__ __forceinline__ void fluid_cell(const uint32_t c, const Acc& P, S* __restrict__ Pout,
+                                           const float* __restrict__ u_in_ptr, float* __restrict__ rho_o,
+                                           float* __restrict__ ux_o, float* __restrict__ uy_o,
+                                           float* __restrict__ uz_o, const StepParams& p, const uint32_t lw,
+                                           float& rho, float& ux, float& uy, float& uz) {
+  float F[kQ];
+  if (link_type(lw) == kFluid) fluid_gather<S, kLd>(P, lw, F);
+  else fluid_gather_end<S, kLd>(P, u_in_ptr, p, lw, F);
+  fluid_collide<S, kMacro>(c, P, Pout, rho_o, ux_o, uy_o, uz_o, p, F, rho, ux, uy, uz);
 }
 
 // fluid lattice of a solid cell: on macro steps the moments of its frozen populations, which are the rest
@@ -399,22 +445,15 @@ __device__ __forceinline__ void solid_cell(const uint32_t c, float* __restrict__
   }
 }
 
-// thermal lattice of any cell, with the cell's fluid velocity u (0 in solids)
-template <typename S, bool kOwn, int kLd, int kT, class Acc>
-__device__ __forceinline__ void thermal_cell(const uint32_t c, const Acc& Q, S* __restrict__ Qo,
-                                             const float* __restrict__ qsrc, const float* __restrict__ T0,
-                                             const StepParams& p, const uint32_t lw, const float ux, const float uy,
-                                             const float uz) {
+// Thermal populations streamed to a cell (kOwn: its initial ones, unstreamed)
+template <typename S, bool kOwn, int kLd, class Acc>
+__device__ __forceinline__ void thermal_gather(const Acc& Q, const StepParams& p, const uint32_t lw, float (&G)[kQ]) {
   const int type = link_type(lw);
-  const int RL = row_len<kT>(p.g);
   const float Tb = p.T_ref;
-  float G[kQ];
-  float T;
   if (kOwn) {
 #define XAC_LD_G0(I) G[I] = Pop<S>::template ld<kLd>(Q.own(I), w_of(I) * Tb);
     XAC_FOR19(XAC_LD_G0)
 #undef XAC_LD_G0
-    T = kLd == 1 ? __ldcg(T0 + c) : __ldg(T0 + c);  // T0 lives in global memory
   } else {
     if (type == kInlet) {
       // src/thermal_engine3d.py:160-165
@@ -459,6 +498,22 @@ __device__ __forceinline__ void thermal_cell(const uint32_t c, const Acc& Q, S* 
       XAC_FOR19(XAC_LD_GSLOW)
 #undef XAC_LD_GSLOW
     }
+  }
+}
+
+// Temperature and collision of any cell, with the cell's fluid velocity u (0 in solids; kRest: 0 in every lane of the warp;
+// kHeat false: no lane of the warp is heated)
+template <typename S, bool kOwn, int kLd, int kT, bool kRest = false, bool kHeat = true>
+__device__ __forceinline__ void thermal_collide(const uint32_t c, S* __restrict__ Qo, const float* __restrict__ qsrc,
+                                                const float* __restrict__ T0, const StepParams& p, const uint32_t lw,
+                                                const float (&G)[kQ], const float ux, const float uy,
+                                                const float uz) {
+  const int type = link_type(lw);
+  const float Tb = p.T_ref;
+  float T;
+  if (kOwn) {
+    T = kLd == 1 ? __ldcg(T0 + c) : __ldg(T0 + c);  // T0 lives in global memory
+  } else {
     // src/thermal_engine3d.py:214-224
     T = 0.0f;
 #pragma unroll
@@ -468,17 +523,42 @@ __device__ __forceinline__ void thermal_cell(const uint32_t c, const Acc& Q, S* 
   const bool solid = type == kSolid;
   const float omega_t = solid ? p.omega_ts : p.omega_tf;
   const float srcf = solid ? p.srcf_s : p.srcf_f;
-  const float q = (lw & kHeatedBit) ? __ldg(qsrc + c) : 0.0f;
-  const float usq15t = 1.5f * ((ux * ux + uy * uy) + uz * uz);
-#define XAC_TCOLLIDE(I)                                                          \
+  const bool heated = kHeat && (lw & kHeatedBit);
+  const float q = heated ? __ldg(qsrc + c) : 0.0f;
+#define XAC_TOUT(I, GE)                                                          \
   {                                                                              \
-    const float ge = feq_term(w_of(I) * T, edotu<I>(ux, uy, uz), usq15t);       \
-    float v = G[I] - omega_t * (G[I] - ge);                                      \
-    if (q > 0.0f) v += (w_of(I) * srcf) * q;                                     \
-    Pop<S>::st(Qo + (I) * RL, v, w_of(I) * Tb);                                \
+    float v = G[I] - omega_t * (G[I] - (GE));                                    \
+    if (heated && q > 0.0f) v += (w_of(I) * srcf) * q;                           \
+    Pop<S>::st(Qo + (kT > 0 ? (uint32_t)((I) * kT) : p.g.own_off[I]), v, w_of(I) * Tb); \
   }
-  XAC_FOR19(XAC_TCOLLIDE)
-#undef XAC_TCOLLIDE
+  if (kRest) {  // u = 0: every bracket of the equilibrium is exactly 1
+#define XAC_TREST(I) XAC_TOUT(I, w_of(I) * T)
+    XAC_FOR19(XAC_TREST)
+#undef XAC_TREST
+  } else {
+    const float usq15t = 1.5f * ((ux * ux + uy * uy) + uz * uz);
+    XAC_TOUT(0, (w_of(0) * T) * (1.0f - usq15t))
+#define XAC_TPAIR(I, J)                                                          \
+  {                                                                              \
+    float gi, gj;                                                                \
+    feq_pair(w_of(I) * T, edotu<I>(ux, uy, uz), usq15t, gi, gj);                 \
+    XAC_TOUT(I, gi)                                                              \
+    XAC_TOUT(J, gj)                                                              \
+  }
+    XAC_PAIRS(XAC_TPAIR)
+#undef XAC_TPAIR
+  }
+#undef XAC_TOUT
+}
+
+template <typename S, bool kOwn, int kLd, int kT, class Acc>
+__device__ __forceinline__ void thermal_cell(const uint32_t c, const Acc& Q, S* __restrict__ Qo,
+                                             const float* __restrict__ qsrc, const float* __restrict__ T0,
+                                             const StepParams& p, const uint32_t lw, const float ux, const float uy,
+                                             const float uz) {
+  float G[kQ];
+  thermal_gather<S, kOwn, kLd>(Q, p, lw, G);
+  thermal_collide<S, kOwn, kLd, kT>(c, Qo, qsrc, T0, p, lw, G, ux, uy, uz);
 }
 
 // cell c = (row r, x); its thermal populations start at element e0; SP / SQ: fluid / thermal storage
@@ -493,10 +573,10 @@ __device__ __forceinline__ void coupled_cell(const uint32_t c, const uint32_t r,
                                              const uint32_t lw) {
   const int RL = row_len<kT>(p.g);
   const bool fluid = valid && link_type(lw) != kSolid;
-  float ux = 0.0f, uy = 0.0f, uz = 0.0f;
+  float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
   if (fluid) {
     const FluidAt<SP> P = fluid_at(Pin, r, x, p.g, p.ftab);
-    fluid_cell<SP, kMacro, kLd>(c, P, Pout + P.k, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, ux, uy, uz);
+    fluid_cell<SP, kMacro, kLd>(c, P, Pout, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, rho, ux, uy, uz);
   } else if (valid) {
     solid_cell<kMacro>(c, rho_o, ux_o, uy_o, uz_o);
   }
@@ -517,31 +597,136 @@ __device__ __forceinline__ void pad_fill(bool valid, unsigned valid_lanes, int l
   }
 }
 
-// One thread per row position: block-consecutive threads walk x along a row (a warp never spans two rows, the
-// row length being a multiple of 32); positions x >= nx are padding. kT > 0 makes the row length and every
-// thermal population offset compile-time constants; kT = 0 reads it from the geometry.
-template <typename SP, typename SQ, bool kMacro, bool kOwn, int kT>
-__global__ void __launch_bounds__(256) coupled_step_kernel(const SP* __restrict__ Pin, SP* __restrict__ Pout,
-                                                           const SQ* __restrict__ Qin, SQ* __restrict__ Qout,
-                                                           const uint32_t* __restrict__ link,
-                                                           const float* __restrict__ qsrc,
-                                                           const float* __restrict__ u_in_ptr,
-                                                           float* __restrict__ rho_o, float* __restrict__ ux_o,
-                                                           float* __restrict__ uy_o, float* __restrict__ uz_o,
-                                                           const float* __restrict__ T0, StepParams p) {
-  const int RL = row_len<kT>(p.g);
-  const uint32_t blk = p.reverse ? gridDim.x - 1u - blockIdx.x : blockIdx.x;
-  const uint32_t pos = blk * blockDim.x + threadIdx.x;
+// ---- the two lattices side by side (launch variant 0) ----------------------------------------------------
+// The fluid does not depend on the temperature, so the lattices run as two kernels, the fluid's a step ahead: fluid step
+// k + 1 beside thermal step k, on two branches of the captured graph. The fluid kernel takes the non-solid cells in storage
+// order, one per thread: its warps are full, where a warp of 32 consecutive x has 43% non-solid lanes on a 57%-solid
+// gyroid. The thermal kernel takes one row position per thread and reads u by slot from one of two sets.
+// Bound: memory in FP32 (152 B per cell and 152 B per non-solid cell, and 24 B per non-solid cell for u; a plain
+// ping-pong copy of those bytes takes 21.5 us on the 148x128x32 gyroid), instruction issue in 16 bits (9.4 M + 6.2 M
+// warp instructions a step, where one pass over the row positions takes 21.8 M + conversions). Measured on that design, one
+// kernel for both lattices by row position -> this: FP32 28.5 -> 27.0 us, FP16 28.8 -> 20.5, FP32 fluid with FP16
+// thermal 27.2 -> 21.5. Tried: both lattices in one launch, fluid blocks first 33.4 (more DRAM traffic: the thermal rows of the
+// last step have left L2), with u in cell order 29.3, programmatic dependent launch -2% to +10%, thermal rows staged in
+// shared memory 27.7 / 21.7, 32 registers 28.6 / 22.6, both in one launch with alternating blocks 28.9 / 23.9.
+struct SplitArgs {
+  const void* Pin;  // fluid step k + 1
+  void* Pout;
+  const void* Qin;  // thermal step k
+  void* Qout;
+  const uint32_t* link;
+  const float* qsrc;
+  const float* u_in;
+  const uint2* cells;    // per non-solid cell: link word with x & 31 from bit 24, table entry of its word
+  const uint32_t* ends;  // slots of the inlet and outlet cells
+  float* field[4];       // rho, u; field[0] not null: the fluid step writes those of its cells
+  float* uo[3];          // u of step k + 1
+  const float* ui[3];    // u of step k
+  float* solid[4];       // solid[0] not null: the thermal step writes rho, u of the solid cells
+  const float* T0;
+  uint32_t nfluid, nends;       // non-solid cells; inlet and outlet cells among them
+  uint32_t fblocks, eblocks;    // blocks of non-solid cells, blocks of the inlet and outlet cells (0: no fluid step)
+  uint32_t tblocks;             // blocks of the thermal step
+  uint32_t frev, trev;          // blocks in reverse order
+  int own;                      // the thermal step reads its populations unstreamed (first step)
+  StepParams p;
+};
+
+constexpr int kCellXShift = 24;
+constexpr uint32_t kCellXMask = 31u << kCellXShift;
+
+// cell index of a non-solid cell from its table entry and x & 31
+__device__ __forceinline__ uint32_t cell_of_entry(const Geom& g, uint32_t t0, uint32_t x31) {
+  const uint32_t nt = (uint32_t)g.nt;
+  const uint32_t row = t0 / nt, w = t0 - row * nt;
+  return (row - (uint32_t)g.ny - 1u) * (uint32_t)g.nx + w * 32u + x31;
+}
+
+// the non-solid cell in slot k; kEnd: an inlet or outlet cell (the blocks of the other cells leave those out, so a warp
+// runs one of the two gathers)
+template <typename SP, bool kPlain, bool kEnd>
+__device__ __forceinline__ void split_fluid(const SplitArgs& a, const uint32_t k) {
+  const uint2 info = __ldg(a.cells + k);
+  const uint32_t lw = info.x & ~kCellXMask, x31 = (info.x & kCellXMask) >> kCellXShift;
+  if (!kEnd && link_type(lw) != kFluid) return;
+  FluidAt<SP> P;
+  float F[kQ];
+  if (kEnd) {
+    P.base = (const SP*)a.Pin;
+    P.run = a.p.g.run;
+    P.k = k;
+    fluid_gather_end<SP, 0>(P, a.u_in, a.p, lw, F);
+  } else {
+    P = fluid_at_entry<SP>((const SP*)a.Pin, k, info.y, x31, a.p.g, a.p.ftab);
+    fluid_gather<SP, 0>(P, lw, F);
+  }
+  float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
+  fluid_collide<SP, false>(0u, P, (SP*)a.Pout, nullptr, nullptr, nullptr, nullptr, a.p, F, rho, ux, uy, uz);
+  a.uo[0][k] = ux;
+  a.uo[1][k] = uy;
+  a.uo[2][k] = uz;
+  if (!kPlain && a.field[0]) {
+    const uint32_t c = cell_of_entry(a.p.g, info.y, x31);
+    a.field[0][c] = rho;
+    a.field[1][c] = ux;
+    a.field[2][c] = uy;
+    a.field[3][c] = uz;
+  }
+}
+
+template <typename SQ, bool kPlain, int kT>
+__device__ __forceinline__ void split_thermal(const SplitArgs& a, const uint32_t pos) {
+  const Geom& g = a.p.g;
+  const int RL = row_len<kT>(g);
   const uint32_t r = pos / (uint32_t)RL, x = pos - r * (uint32_t)RL;
-  if (r >= (uint32_t)p.g.rows) return;  // whole warps
+  if (r >= (uint32_t)g.rows) return;  // whole warps (the row length is a multiple of 32)
   const int lane = threadIdx.x & 31;
-  const bool valid = x < (uint32_t)p.g.nx;
-  const uint32_t c = r * (uint32_t)p.g.nx + x;
-  const uint32_t lw = valid ? __ldg(link + c) : ((uint32_t)kSolid << kTypeShift);
-  const uint32_t e0 = pop_base(r, x, p.g, RL);
-  coupled_cell<SP, SQ, kMacro, kOwn, 0, kT>(c, r, x, e0, Pin, Pout, Qin, Qout, qsrc, u_in_ptr, rho_o, ux_o, uy_o,
-                                            uz_o, T0, p, valid, lw);
-  pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, Qout, e0, p.g);
+  const bool valid = x < (uint32_t)g.nx;
+  const uint32_t c = r * (uint32_t)g.nx + x;
+  const uint32_t lw = valid ? __ldg(a.link + c) : ((uint32_t)kSolid << kTypeShift);
+  const uint32_t e0 = pop_base(r, x, g, RL);
+  const bool fluid = link_type(lw) != kSolid;
+  const bool moving = __any_sync(0xffffffffu, fluid), heated = __any_sync(0xffffffffu, (lw & kHeatedBit) != 0u);
+  if (valid) {
+    const Rows<SQ, kT> Q = rows_at<kT>((const SQ*)a.Qin, e0, g, RL);
+    SQ* Qo = (SQ*)a.Qout + e0;
+    // the populations are on their way while the cell's slot and then its velocity are looked up
+    const uint2 e = __ldg(a.p.ftab + ftab_index(g, r, x));
+    float G[kQ];
+    if (!kPlain && a.own) thermal_gather<SQ, true, 0>(Q, a.p, lw, G);
+    else thermal_gather<SQ, false, 0>(Q, a.p, lw, G);
+    float ux = 0.0f, uy = 0.0f, uz = 0.0f;
+    if (fluid) {
+      const uint32_t k = e.y + (uint32_t)__popc(e.x & ((1u << (x & 31u)) - 1u));
+      ux = __ldg(a.ui[0] + k);
+      uy = __ldg(a.ui[1] + k);
+      uz = __ldg(a.ui[2] + k);
+    }
+    if (!kPlain && a.own) thermal_collide<SQ, true, 0, kT>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
+    else if (heated) thermal_collide<SQ, false, 0, kT>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
+    else if (moving) thermal_collide<SQ, false, 0, kT, false, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
+    else thermal_collide<SQ, false, 0, kT, true, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
+    if (!kPlain && a.solid[0] && !fluid) solid_cell<true>(c, a.solid[0], a.solid[1], a.solid[2], a.solid[3]);
+  }
+  pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, (SQ*)a.Qout, e0, g);
+}
+
+// kPlain: no first step and no field output in this launch
+template <typename SP, bool kPlain>
+__global__ void __launch_bounds__(256) split_fluid_kernel(const __grid_constant__ SplitArgs a) {
+  const uint32_t b = blockIdx.x;
+  if (b < a.fblocks) {
+    const uint32_t k = (a.frev ? a.fblocks - 1u - b : b) * blockDim.x + threadIdx.x;
+    if (k < a.nfluid) split_fluid<SP, kPlain, false>(a, k);
+    return;
+  }
+  const uint32_t i = (b - a.fblocks) * blockDim.x + threadIdx.x;
+  if (i < a.nends) split_fluid<SP, kPlain, true>(a, __ldg(a.ends + i));
+}
+template <typename SQ, bool kPlain, int kT>
+__global__ void __launch_bounds__(256) split_thermal_kernel(const __grid_constant__ SplitArgs a) {
+  const uint32_t b = blockIdx.x;
+  split_thermal<SQ, kPlain, kT>(a, (a.trev ? a.tblocks - 1u - b : b) * blockDim.x + threadIdx.x);
 }
 
 // ---- thermal rows staged in shared memory (launch variant 1) ------------------------------------------
@@ -625,10 +810,10 @@ __global__ void __launch_bounds__(kT) coupled_qstage_kernel(const SP* __restrict
   const uint32_t c = r * (uint32_t)p.g.nx + x;
   const uint32_t lw = valid ? __ldg(link + c) : ((uint32_t)kSolid << kTypeShift);
   const uint32_t e0 = pop_base(r, x, p.g, kT);
-  float ux = 0.0f, uy = 0.0f, uz = 0.0f;
+  float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
   if (valid && link_type(lw) != kSolid) {
     const FluidAt<SP> P = fluid_at(Pin, r, x, p.g, p.ftab);
-    fluid_cell<SP, kMacro, 0>(c, P, Pout + P.k, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, ux, uy, uz);
+    fluid_cell<SP, kMacro, 0>(c, P, Pout, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, rho, ux, uy, uz);
   } else if (valid) {
     solid_cell<kMacro>(c, rho_o, ux_o, uy_o, uz_o);
   }
@@ -640,8 +825,8 @@ __global__ void __launch_bounds__(kT) coupled_qstage_kernel(const SP* __restrict
   pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, Qout, e0, p.g);
 }
 
-// Arguments of one fused step launch; launch_coupled_step<SP, SQ> (step_kernels.cuh, one translation unit per
-// storage mode) picks the instantiation whose compile-time row length matches the lattice.
+// Arguments of one staged step launch; the launchers (step_kernels.cuh, one translation unit per storage mode) pick the
+// instantiation whose compile-time row length matches the lattice.
 struct StepLaunch {
   const void* Pin;
   void* Pout;
@@ -653,13 +838,18 @@ struct StepLaunch {
   float *rho, *ux, *uy, *uz;
   const float* T0;
   StepParams p;
-  int block;
-  int variant;  // 0: one thread per row position; 1: thermal rows staged in shared memory (compile-time pitch)
   bool macro, own;
   cudaStream_t stream;
 };
+// the staged step (variant 1; row lengths up to kMaxStagedRow)
+constexpr int kMaxStagedRow = 320;
 template <typename SP, typename SQ>
-void launch_coupled_step(const StepLaunch& a);
+void launch_staged_step(const StepLaunch& a);
+// the two halves of the split step (variant 0); plain: no first step and no field output
+template <typename SP>
+void launch_split_fluid(const SplitArgs& a, int block, bool plain, cudaStream_t s);
+template <typename SQ>
+void launch_split_thermal(const SplitArgs& a, int block, bool plain, cudaStream_t s);
 
 // omega and source factors, computed with the device's IEEE division once per lattice
 static __global__ void relaxation_factors_kernel(float tau_f, float tau_tf, float tau_ts, float* out) {

@@ -3,5 +3,6 @@
 #include "step_kernels.cuh"
 
 namespace xac {
-template void launch_coupled_step<__nv_bfloat16, __half>(const StepLaunch&);
+template void launch_staged_step<__nv_bfloat16, __half>(const StepLaunch&);
+template void launch_split_fluid<__nv_bfloat16>(const SplitArgs&, int, bool, cudaStream_t);
 }  // namespace xac

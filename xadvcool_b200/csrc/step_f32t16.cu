@@ -2,5 +2,5 @@
 #include "step_kernels.cuh"
 
 namespace xac {
-template void launch_coupled_step<float, __half>(const StepLaunch&);
+template void launch_staged_step<float, __half>(const StepLaunch&);
 }  // namespace xac

@@ -59,6 +59,14 @@ __device__ __forceinline__ float feq_term(float w_rho, float eu, float usq15) {
   return w_rho * (((1.0f + 3.0f * eu) + 4.5f * (eu * eu)) - usq15);
 }
 
+// The same for a direction (e_i . u = eu) and its opposite (-eu): 1 + 3(-eu) is 1 - 3eu and (-eu)^2 is eu^2 exactly, so both
+// carry the bits of feq_term.
+__device__ __forceinline__ void feq_pair(float w_rho, float eu, float usq15, float& fi, float& fj) {
+  const float t = 3.0f * eu, q = 4.5f * (eu * eu);
+  fi = w_rho * (((1.0f + t) + q) - usq15);
+  fj = w_rho * (((1.0f - t) + q) - usq15);
+}
+
 // Thread-local error message behind xac_last_error().
 void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* what);
