@@ -343,6 +343,20 @@ int xac_conv3d_partial_floats(int N, int D, int H, int W, int Ci, int Co, int ks
 /* Reads and clears the device-side status of the convolution kernels (synchronises the device): bit 0 set means a
  * bounded wait inside a tensor-core kernel ran out, and that launch left its output unwritten. */
 int xac_conv3d_status(int *flags);
+/* out = GELU(gamma h + beta), h = (y - mean) rstd, mean and rstd [N][G] over V voxels and C/G channels; BF16 [N][V][C]
+ * in and out, FP32 between, every operation rounded by itself. C a power of two (8..256), C/G a multiple of 4, volumes
+ * 16-byte aligned. Backward: grad_terms gives dgamma, dbeta and the FP32 volumes direct = dh rstd and slope = dh (y - mean),
+ * dh the gradient of h; backward gives dy = direct + k2 (y - mean) + k1 (BF16) from the two [N][G] parts that the caller
+ * derives from the groups' sums of slope and direct. scratch: xac_norm_act_scratch_doubles() doubles. Deterministic. */
+int xac_norm_act_forward(const void *y, int N, long long V, int C, int G, const float *mean, const float *rstd,
+                         const float *gamma, const float *beta, void *out, void *stream);
+int xac_norm_act_grad_terms(const void *y, const void *d_out, int N, long long V, int C, int G, const float *mean,
+                            const float *rstd, const float *gamma, const float *beta, double *scratch, float *direct,
+                            float *slope, float *dgamma, float *dbeta, void *stream);
+int xac_norm_act_backward(const void *y, const void *d_out, int N, long long V, int C, int G, const float *mean,
+                          const float *rstd, const float *gamma, const float *beta, const float *k1, const float *k2,
+                          void *dy, void *stream);
+int xac_norm_act_scratch_doubles(int N, long long V, int C, int G, long long *count);
 
 /* ========================================================================== *
  * Design generator on the device: the seeded benchmark families of xadvcool_b200.designs (gyroid_design,

@@ -136,6 +136,10 @@ SIGNATURES = {
     "xac_conv3d_weight_grad": [_vp, _i, _i, _i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _vp],
     "xac_conv3d_partial_floats": [_i, _i, _i, _i, _i, _i, _i, C.POINTER(C.c_longlong)],
     "xac_conv3d_status": [C.POINTER(_i)],
+    "xac_norm_act_forward": [_vp, _i, C.c_longlong, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp],
+    "xac_norm_act_grad_terms": [_vp, _vp, _i, C.c_longlong, _i, _i] + [_vp] * 10,
+    "xac_norm_act_backward": [_vp, _vp, _i, C.c_longlong, _i, _i] + [_vp] * 8,
+    "xac_norm_act_scratch_doubles": [_i, C.c_longlong, _i, _i, C.POINTER(C.c_longlong)],
     "xac_batch_create": [C.POINTER(Desc), _i, C.POINTER(_vp), _vp],
     "xac_batch_destroy": [_vp],
     "xac_batch_size": [_vp, C.POINTER(_i)],

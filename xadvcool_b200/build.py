@@ -31,6 +31,7 @@ UNITS = [
     ("step_f32t16.cu", ["--fmad=false"]),
     ("stats_noalloc.cu", ["--fmad=false"]),
     ("conv3d.cu", []),
+    ("norm_act.cu", []),
     ("designs.cu", ["--fmad=false"]),
 ]
 

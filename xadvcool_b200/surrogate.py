@@ -5,9 +5,9 @@ Architecture (after the reference's 3-D U-Net, benchmark/models/unet3d.py:11-125
 16, 32, 64, 128 channels, two 3x3x3 convolution - GroupNorm - GELU units per level (unet3d.py:11-26), 2x
 average pooling down, nearest 2x upsampling + skip concatenation up, and a 1x1 head. Weights are kept in FP32
 (the optimiser's copy) and run in BF16. Every convolution - forward, data gradient and weight gradient - is
-libxac.so's BF16 tensor-core implicit GEMM with FP32 accumulation (csrc/conv3d.cu). GroupNorm, pooling,
-upsampling, concatenation, GELU, the loss and AdamW (benchmark/train.py:128-141) are torch tensor operations
-around those kernels.
+libxac.so's BF16 tensor-core implicit GEMM with FP32 accumulation (csrc/conv3d.cu), and GroupNorm with GELU is one
+fused pass of its own (csrc/norm_act.cu). Pooling, upsampling, concatenation, the loss and AdamW
+(benchmark/train.py:128-141) are torch tensor operations around those kernels.
 
 Volumes are channels-last, [batch][z][y][x][channel], x padded from 148 to 152 so three poolings divide it.
 """
@@ -125,6 +125,88 @@ def torch_conv3d(x, w, b, ksize=3, out_fp32=False):
     return y if out_fp32 else y.to(BF16)
 
 
+# ------------------------------------------------------------------------------------------------ GroupNorm + GELU
+EPS = 1e-5
+
+
+def _group_stats(y, groups):
+    """(centred source, mean, 1/std) of the groups: y in FP32 as [N, voxels, groups, channels of a group]"""
+    h = y.float().reshape(y.shape[0], -1, groups, y.shape[-1] // groups)
+    mean = h.mean(dim=(1, 3), keepdim=True)
+    var = h.var(dim=(1, 3), unbiased=False, keepdim=True)
+    return h, mean, torch.rsqrt(var + EPS)
+
+
+def norm_gelu(y, g, s, groups):
+    """GroupNorm over channels-last volumes [N,D,H,W,C], scale g, shift s, GELU; FP32 inside, BF16 out: tensor
+    operations, on any device."""
+    h, mean, rstd = _group_stats(y, groups)
+    h = ((h - mean) * rstd).reshape(y.shape)
+    return F.gelu(h * g + s).to(BF16)
+
+
+def _aligned(t):
+    """Contiguous, on a 16-byte boundary, as the kernels' wide loads need it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _norm_act_takes(y, g, s, groups) -> bool:
+    """The calls the fused kernels are written for (csrc/norm_act.cu): BF16 volumes with FP32 scale and shift, a power of
+    two of channels up to 256 (octets of channels divide a warp) in groups of a multiple of 4 (half an octet)."""
+    C = y.shape[-1]
+    return (y.is_cuda and y.dtype == BF16 and y.numel() > 0 and y.shape[0] <= 65535 and y.numel() // (y.shape[0] * C) <= 2 ** 31
+            and 8 <= C <= 256 and C & (C - 1) == 0 and C % groups == 0 and C // groups % 4 == 0
+            and all(p.dtype == torch.float32 and p.device == y.device and p.shape == (C,) for p in (g, s)))
+
+
+class _NormAct(torch.autograd.Function):
+    """norm_gelu with everything after the groups' statistics in one pass (csrc/norm_act.cu). The statistics stay tensor
+    operations, and so do the groups' sums of the gradient: how single BF16 values round hangs on the FP32 sums, and all
+    other layers carry that on."""
+
+    @staticmethod
+    def forward(ctx, y, g, s, groups):
+        N, Cc = y.shape[0], y.shape[-1]
+        _, mean, rstd = _group_stats(y, groups)
+        ctx.save_for_backward(y, g, s, mean, rstd)
+        ctx.groups = groups
+        y, g, s = _aligned(y), g.contiguous(), s.contiguous()
+        out = torch.empty_like(y)
+        _capi.call("xac_norm_act_forward", y.data_ptr(), N, y.numel() // (N * Cc), Cc, groups, mean.data_ptr(),
+                   rstd.data_ptr(), g.data_ptr(), s.data_ptr(), out.data_ptr(), stream_ptr(y.device))
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        y, g, s, mean, rstd = ctx.saved_tensors
+        if torch.is_grad_enabled():  # a graph of the gradient is wanted: the same gradient by tensor operations
+            need = [t for t, n in zip((y, g, s), ctx.needs_input_grad) if n]
+            grads = iter(torch.autograd.grad(norm_gelu(y, g, s, ctx.groups), need, dout, create_graph=True))
+            return tuple(next(grads) if n else None for n in ctx.needs_input_grad[:3]) + (None,)
+        y, dout, g, s, mean, rstd = _aligned(y), _aligned(dout), *(t.contiguous() for t in (g, s, mean, rstd))
+        N, Cc = y.shape[0], y.shape[-1]
+        V = y.numel() // (N * Cc)
+        cnt = C.c_longlong()
+        _capi.call("xac_norm_act_scratch_doubles", N, V, Cc, ctx.groups, C.byref(cnt))
+        scratch = torch.empty(int(cnt.value), dtype=torch.float64, device=y.device)
+        direct, slope = (torch.empty((N, V, ctx.groups, Cc // ctx.groups), dtype=torch.float32, device=y.device)
+                         for _ in range(2))
+        dg, ds = torch.empty_like(g), torch.empty_like(s)
+        _capi.call("xac_norm_act_grad_terms", y.data_ptr(), dout.data_ptr(), N, V, Cc, ctx.groups, mean.data_ptr(),
+                   rstd.data_ptr(), g.data_ptr(), s.data_ptr(), scratch.data_ptr(), direct.data_ptr(), slope.data_ptr(),
+                   dg.data_ptr(), ds.data_ptr(), stream_ptr(y.device))
+        M = V * (Cc // ctx.groups)
+        dvar = -0.5 * slope.sum(dim=(1, 3), keepdim=True) * rstd.pow(3)
+        k1, k2 = -direct.sum(dim=(1, 3), keepdim=True) / M, (2.0 / M) * dvar
+        del direct, slope
+        dy = torch.empty_like(y)
+        _capi.call("xac_norm_act_backward", y.data_ptr(), dout.data_ptr(), N, V, Cc, ctx.groups, mean.data_ptr(),
+                   rstd.data_ptr(), g.data_ptr(), s.data_ptr(), k1.data_ptr(), k2.data_ptr(), dy.data_ptr(),
+                   stream_ptr(y.device))
+        return dy, dg, ds, None
+
+
 # ------------------------------------------------------------------------------------------------ model
 class Surrogate:
     """The encoder-decoder; parameters are FP32 tensors (w: [taps, Co, Ci], b: [Co])."""
@@ -174,13 +256,12 @@ class Surrogate:
     def _unit(self, x, name, conv):
         """conv -> GroupNorm -> GELU, channels-last, normalisation in FP32."""
         y = conv(x, self.params[name + ".w"], self.params[name + ".b"], 3, False)
-        N, C = y.shape[0], y.shape[-1]
-        G = self.groups(C)
-        h = y.float().reshape(N, -1, G, C // G)
-        mean = h.mean(dim=(1, 3), keepdim=True)
-        var = h.var(dim=(1, 3), unbiased=False, keepdim=True)
-        h = ((h - mean) * torch.rsqrt(var + 1e-5)).reshape(y.shape)
-        return F.gelu(h * self.params[name + ".g"] + self.params[name + ".s"]).to(BF16)
+        g, s, G = self.params[name + ".g"], self.params[name + ".s"], self.groups(y.shape[-1])
+        # beside the tensor-core convolutions (which have no forward mode, vmap or host form either) the fused kernels;
+        # under a caller's own convolution the tensor operations, which take all of those
+        if conv is conv3d and _norm_act_takes(y, g, s, G):
+            return _NormAct.apply(y, g, s, G)
+        return norm_gelu(y, g, s, G)
 
     def _block(self, x, name, conv):
         return self._unit(self._unit(x, name + "a", conv), name + "b", conv)
