@@ -357,6 +357,11 @@ int xac_norm_act_backward(const void *y, const void *d_out, int N, long long V, 
                           const float *rstd, const float *gamma, const float *beta, const float *k1, const float *k2,
                           void *dy, void *stream);
 int xac_norm_act_scratch_doubles(int N, long long V, int C, int G, long long *count);
+/* 2x average pooling and nearest 2x upsampling joined to a skip volume, BF16 channels-last, sums in FP32. N, D, H, W are
+ * the coarse volume's extents; the fine one's are N, 2D, 2H, 2W. Channels are multiples of 8, volumes 16-byte aligned and
+ * of at most 2^33 values. xac_pool2: in fine, out coarse; backward: in the coarse gradient, out the fine one. */
+int xac_pool2(const void *in, int N, int D, int H, int W, int C, int backward, void *out, void *stream);
+int xac_upcat2(const void *low, const void *skip, int N, int D, int H, int W, int Ca, int Cb, void *out, void *stream);
 
 /* ========================================================================== *
  * Design generator on the device: the seeded benchmark families of xadvcool_b200.designs (gyroid_design,

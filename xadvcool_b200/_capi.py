@@ -140,6 +140,8 @@ SIGNATURES = {
     "xac_norm_act_grad_terms": [_vp, _vp, _i, C.c_longlong, _i, _i] + [_vp] * 10,
     "xac_norm_act_backward": [_vp, _vp, _i, C.c_longlong, _i, _i] + [_vp] * 8,
     "xac_norm_act_scratch_doubles": [_i, C.c_longlong, _i, _i, C.POINTER(C.c_longlong)],
+    "xac_pool2": [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "xac_upcat2": [_vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "xac_batch_create": [C.POINTER(Desc), _i, C.POINTER(_vp), _vp],
     "xac_batch_destroy": [_vp],
     "xac_batch_size": [_vp, C.POINTER(_i)],

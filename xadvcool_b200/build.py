@@ -32,6 +32,7 @@ UNITS = [
     ("stats_noalloc.cu", ["--fmad=false"]),
     ("conv3d.cu", []),
     ("norm_act.cu", []),
+    ("resample.cu", []),
     ("designs.cu", ["--fmad=false"]),
 ]
 

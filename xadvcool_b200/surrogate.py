@@ -6,8 +6,9 @@ Architecture (after the reference's 3-D U-Net, benchmark/models/unet3d.py:11-125
 average pooling down, nearest 2x upsampling + skip concatenation up, and a 1x1 head. Weights are kept in FP32
 (the optimiser's copy) and run in BF16. Every convolution - forward, data gradient and weight gradient - is
 libxac.so's BF16 tensor-core implicit GEMM with FP32 accumulation (csrc/conv3d.cu), and GroupNorm with GELU is one
-fused pass of its own (csrc/norm_act.cu). Pooling, upsampling, concatenation, the loss and AdamW
-(benchmark/train.py:128-141) are torch tensor operations around those kernels.
+fused pass of its own (csrc/norm_act.cu), pooling and upsampling with concatenation one pass each
+(csrc/resample.cu). The groups' statistics, the loss and AdamW (benchmark/train.py:128-141) are torch tensor
+operations around those kernels.
 
 Volumes are channels-last, [batch][z][y][x][channel], x padded from 148 to 152 so three poolings divide it.
 """
@@ -207,6 +208,67 @@ class _NormAct(torch.autograd.Function):
         return dy, dg, ds, None
 
 
+# ------------------------------------------------------------------------------------------------ resolution
+def pool2(x):
+    """2x average pooling of a channels-last volume: tensor operations, on any device."""
+    N, D, H, W, Cc = x.shape
+    return x.view(N, D // 2, 2, H // 2, 2, W // 2, 2, Cc).float().mean(dim=(2, 4, 6)).to(BF16)
+
+
+def up2(x):
+    """Nearest 2x upsampling of a channels-last volume: tensor operations, on any device."""
+    N, D, H, W, Cc = x.shape
+    return x[:, :, None, :, None, :, None, :].expand(N, D, 2, H, 2, W, 2, Cc).reshape(N, 2 * D, 2 * H, 2 * W, Cc)
+
+
+def _resample_takes(*volumes) -> bool:
+    """The calls the resampling kernels are written for (csrc/resample.cu): BF16 volumes on one GPU in octets of channels,
+    with octets and voxels of the fine volume in 32-bit indexes."""
+    return (all(v.is_cuda and v.dtype == BF16 and v.dim() == 5 and v.shape[-1] % 8 == 0 and v.numel() > 0
+                and v.device == volumes[0].device for v in volumes)
+            and 8 * sum(v.numel() for v in volumes) <= 2 ** 33)
+
+
+class _Pool2(torch.autograd.Function):
+    @staticmethod
+    def _call(src, coarse, backward):
+        N, D, H, W, Cc = coarse
+        src = _aligned(src)
+        shape = (N, 2 * D, 2 * H, 2 * W, Cc) if backward else coarse
+        out = torch.empty(shape, dtype=BF16, device=src.device)
+        _capi.call("xac_pool2", src.data_ptr(), N, D, H, W, Cc, backward, out.data_ptr(), stream_ptr(src.device))
+        return out
+
+    @staticmethod
+    def forward(ctx, x):
+        N, D, H, W, Cc = x.shape
+        return _Pool2._call(x, (N, D // 2, H // 2, W // 2, Cc), 0)
+
+    @staticmethod
+    def backward(ctx, dout):
+        if torch.is_grad_enabled():  # a graph of the gradient is wanted
+            return up2((dout.float() / 8.0).to(BF16))
+        return _Pool2._call(dout, tuple(dout.shape), 1)
+
+
+class _UpCat2(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, low, skip):
+        (N, D, H, W, Ca), Cb = low.shape, skip.shape[-1]
+        low, skip = _aligned(low), _aligned(skip)
+        ctx.Ca = Ca
+        out = torch.empty((N, 2 * D, 2 * H, 2 * W, Ca + Cb), dtype=BF16, device=low.device)
+        _capi.call("xac_upcat2", low.data_ptr(), skip.data_ptr(), N, D, H, W, Ca, Cb, out.data_ptr(),
+                   stream_ptr(low.device))
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        N, D, H, W, _ = dout.shape
+        low = dout[..., :ctx.Ca].reshape(N, D // 2, 2, H // 2, 2, W // 2, 2, ctx.Ca).sum(dim=(2, 4, 6))
+        return low, dout[..., ctx.Ca:]
+
+
 # ------------------------------------------------------------------------------------------------ model
 class Surrogate:
     """The encoder-decoder; parameters are FP32 tensors (w: [taps, Co, Ci], b: [Co])."""
@@ -266,15 +328,17 @@ class Surrogate:
     def _block(self, x, name, conv):
         return self._unit(self._unit(x, name + "a", conv), name + "b", conv)
 
+    # beside the tensor-core convolutions the resampling kernels, else tensor operations, as in _unit
     @staticmethod
-    def _pool(x):
-        N, D, H, W, Cc = x.shape
-        return x.view(N, D // 2, 2, H // 2, 2, W // 2, 2, Cc).float().mean(dim=(2, 4, 6)).to(BF16)
+    def _pool(x, conv=None):
+        fused = conv is conv3d and _resample_takes(x) and x.is_contiguous() and not any(n % 2 for n in x.shape[1:4])
+        return _Pool2.apply(x) if fused else pool2(x)
 
     @staticmethod
-    def _up(x):
-        N, D, H, W, Cc = x.shape
-        return x[:, :, None, :, None, :, None, :].expand(N, D, 2, H, 2, W, 2, Cc).reshape(N, 2 * D, 2 * H, 2 * W, Cc)
+    def _up_cat(low, skip, conv=None):
+        fused = (conv is conv3d and _resample_takes(low, skip) and low.shape[0] == skip.shape[0]
+                 and all(2 * a == b for a, b in zip(low.shape[1:4], skip.shape[1:4])))
+        return _UpCat2.apply(low, skip) if fused else torch.cat([up2(low), skip], dim=-1)
 
     def forward(self, x, conv=None):
         """x: [N, 32, 128, 152, 16] bf16 features -> [N, 32, 128, 152, 16] fp32 (first 5 channels used).
@@ -283,12 +347,12 @@ class Surrogate:
         torch stand-in to check the rest of the network against them."""
         conv = conv or conv3d
         e0 = self._block(x, "e0", conv)
-        e1 = self._block(self._pool(e0), "e1", conv)
-        e2 = self._block(self._pool(e1), "e2", conv)
-        b3 = self._block(self._pool(e2), "b3", conv)
-        d2 = self._block(torch.cat([self._up(b3), e2], dim=-1), "d2", conv)
-        d1 = self._block(torch.cat([self._up(d2), e1], dim=-1), "d1", conv)
-        d0 = self._block(torch.cat([self._up(d1), e0], dim=-1), "d0", conv)
+        e1 = self._block(self._pool(e0, conv), "e1", conv)
+        e2 = self._block(self._pool(e1, conv), "e2", conv)
+        b3 = self._block(self._pool(e2, conv), "b3", conv)
+        d2 = self._block(self._up_cat(b3, e2, conv), "d2", conv)
+        d1 = self._block(self._up_cat(d2, e1, conv), "d1", conv)
+        d0 = self._block(self._up_cat(d1, e0, conv), "d0", conv)
         return conv(d0, self.params["head.w"], self.params["head.b"], 1, True)
 
     def state_dict(self):
