@@ -222,7 +222,9 @@ int xac_lattice_init_fields(xac_lattice *lat, const float *rho, const float *u, 
 int xac_lattice_step(xac_lattice *lat, int n, void *stream);
 /* Stats of the current step (same quantities as simulation.py:124-129), FP64, deterministic; synchronises. */
 int xac_lattice_stats(xac_lattice *lat, double out_host[XAC_NSTATS], void *stream);
-/* Current macroscopic fields into caller DEVICE buffers, reference layout; any pointer may be NULL. */
+/* Current macroscopic fields into caller DEVICE buffers, reference layout; any pointer may be NULL. Waits for the stream
+ * when a staged step (xac_lattice_tune) ran since the last call that looked at its status; not inside a stream capture,
+ * where the next call outside reports. */
 int xac_lattice_fields(xac_lattice *lat, float *rho, float *u, float *T, void *stream);
 /* Inlet velocity as seen by the streaming step (simulation.py:62, :146 for the pump controller). */
 int xac_lattice_set_inlet(xac_lattice *lat, double u_inlet, void *stream);
@@ -231,10 +233,10 @@ int xac_lattice_steps_done(const xac_lattice *lat, long long *steps);
 /* Launch shape of the step: threads per block (64, 128, 256) and the variant: 0 = the fluid and the thermal lattice in
  * kernels of their own, the fluid a step ahead; 1 = one block per row for both, its thermal input staged in shared
  * memory by bulk copies while the fluid lattice runs (row lengths up to 320; longer ones run variant 0). A lattice
- * starts with block 64 and the variant its size, storage and mask suggest. Variant 1 waits for its copies with a bounded wait; if a wait ever gives up, the call that sees it
- * (xac_lattice_stats, xac_lattice_run) returns XAC_ETIMEOUT and the lattice refuses every further step, run, stats,
- * fields, scalars, validate and save-state call with XAC_ETIMEOUT until xac_lattice_init_fields or
- * xac_lattice_load_state rewrites its populations. Results do not depend on the shape (every cell runs the same
+ * starts with block 64 and the variant its size, storage and mask suggest. Variant 1 waits for its copies with a bounded
+ * wait; if a wait ever gives up, the next call that hands results to the caller (stats, run, fields, scalars, validate,
+ * save-state) returns XAC_ETIMEOUT, also after a change of variant, and the lattice refuses every further call of those and
+ * step with XAC_ETIMEOUT until xac_lattice_init_fields or xac_lattice_load_state rewrites its populations. Results do not depend on the shape (every cell runs the same
  * arithmetic); xadvcool_b200.autotune picks it. */
 int xac_lattice_tune(xac_lattice *lat, int block, int variant);
 int xac_lattice_get_tune(const xac_lattice *lat, int *block, int *variant);

@@ -341,6 +341,33 @@ struct LatticeImpl {
   // set once the status word was seen non-zero: a staged step gave up on its copies, so the thermal populations it
   // wrote are not the step's; the lattice refuses work until init_fields / load_state rewrites its populations
   bool failed = false;
+  // A staged step was launched since the word was last read, whatever the variant is now; steps that a caller captured run
+  // whenever the caller replays them, so after those the word is read every time.
+  bool unread = false, captured_steps = false;
+  bool must_read() const { return unread || captured_steps; }
+  cudaError_t note_staged(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(s, &st);
+    unread = true;
+    captured_steps |= st != cudaStreamCaptureStatusNone;
+    return e;
+  }
+  // the word to host_out, behind what the caller has queued; read_status after the caller's synchronisation
+  cudaError_t copy_status(cudaStream_t s) {
+    if (!must_read()) return cudaSuccess;
+    return cudaMemcpyAsync(host_out + kStatusSlot, red_out + kStatusSlot, sizeof(double), cudaMemcpyDeviceToHost, s);
+  }
+  int read_status(const char* fn) {
+    if (!must_read()) return XAC_OK;
+    unread = false;
+    unsigned st = 0;
+    std::memcpy(&st, host_out + kStatusSlot, sizeof(st));
+    if (st == 0) return XAC_OK;
+    failed = true;
+    set_error("%s: a staged step kernel gave up waiting for its copies (status %u); the lattice refuses further work until "
+              "init_fields or load_state", fn, st);
+    return XAC_ETIMEOUT;
+  }
   int refuse(const char* fn) const {
     set_error("%s: this lattice stopped being usable when a staged step kernel gave up waiting for its copies; "
               "re-initialise it (init_fields) or load a saved state", fn);
@@ -602,6 +629,7 @@ struct LatticeImpl {
   static constexpr int kGraphSteps = 512;
   int steps(int n, cudaStream_t s) {
     if (n <= 0) return XAC_OK;
+    if (staged()) XAC_CUDA(note_staged(s));
     if (own_pending) {
       launch_steps(s, 1, true);
       own_pending = false;
@@ -1041,7 +1069,7 @@ int xac_lattice_init_fields(xac_lattice* lat, const float* rho, const float* u, 
   std::lock_guard<std::mutex> g(lat->impl.mu);
   LatticeImpl& L = lat->impl;
   XAC_CUDA(cudaMemsetAsync(L.status, 0, sizeof(unsigned), as_stream(stream)));
-  L.failed = false;
+  L.failed = L.unread = false;
   return init_impl(L, rho, u, T, as_stream(stream));
 }
 
@@ -1051,6 +1079,7 @@ int xac_test_set_step_status(xac_lattice* lat, unsigned value, void* stream) {
   cudaStream_t s = as_stream(stream);
   XAC_CUDA(cudaMemcpyAsync(lat->impl.status, &value, sizeof(value), cudaMemcpyHostToDevice, s));
   XAC_CUDA(cudaStreamSynchronize(s));
+  lat->impl.unread = true;
   return XAC_OK;
 }
 
@@ -1070,20 +1099,10 @@ int xac_lattice_stats(xac_lattice* lat, double* out_host, void* stream) {
   cudaStream_t s = as_stream(stream);
   int r = L.finalize_T(s);
   if (r != XAC_OK) return r;
-  r = run_stats(L.view(), L.rows, L.red_out, L.host_out, s, L.staged() ? kStatusSlot + 1 : kNStats);
+  r = run_stats(L.view(), L.rows, L.red_out, L.host_out, s, L.must_read() ? kStatusSlot + 1 : kNStats);
   if (r != XAC_OK) return r;
   std::memcpy(out_host, L.host_out, kNStats * sizeof(double));
-  if (L.staged()) {  // the staged kernel's bounded wait reports here
-    unsigned st = 0;
-    std::memcpy(&st, L.host_out + kStatusSlot, sizeof(st));
-    if (st) {
-      L.failed = true;
-      set_error("xac_lattice_stats: a staged step kernel gave up waiting for its copies (status %u); the lattice "
-                "refuses further work until init_fields or load_state", st);
-      return XAC_ETIMEOUT;
-    }
-  }
-  return XAC_OK;
+  return L.read_status("xac_lattice_stats");
 }
 
 int xac_lattice_fields(xac_lattice* lat, float* rho, float* u, float* T, void* stream) {
@@ -1098,7 +1117,13 @@ int xac_lattice_fields(xac_lattice* lat, float* rho, float* u, float* T, void* s
   }
   export_fields_kernel<<<grid_for(L.g.ncell, kBlock), kBlock, 0, s>>>(L.rho, L.ux, L.uy, L.uz, L.T, rho, u, T, L.g);
   XAC_CUDA(cudaGetLastError());
-  return XAC_OK;
+  if (!L.must_read()) return XAC_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  XAC_CUDA(cudaStreamIsCapturing(s, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return XAC_OK;  // a replay's status is for the next call outside the capture
+  XAC_CUDA(L.copy_status(s));
+  XAC_CUDA(cudaStreamSynchronize(s));
+  return L.read_status("xac_lattice_fields");
 }
 
 int xac_lattice_set_inlet(xac_lattice* lat, double u_inlet, void* stream) {
@@ -1201,7 +1226,9 @@ int xac_lattice_scalars(xac_lattice* lat, const xac_scalar_params* prm, double* 
   int r = L.finalize_T(s);
   if (r != XAC_OK) return r;
   MetricBox b{prm->buf, prm->core_nx, prm->core_ny};
+  XAC_CUDA(L.copy_status(s));
   r = run_metrics(L.view(), b, L.rows, L.red_blocks, L.red_out, L.host_out, s);
+  if (r == XAC_OK) r = L.read_status("xac_lattice_scalars");
   if (r != XAC_OK) return r;
   assemble_scalars(L.host_out, L.g.nx, L.g.ny, L.g.nz, prm->buf, prm->t_inlet, prm->tau_fluid, prm->Pr,
                    prm->u_inlet, out_host);
@@ -1224,9 +1251,10 @@ int xac_lattice_validate(xac_lattice* lat, double* out_host, void* stream) {
   combine_rows_kernel<kNValidate><<<1, 32 * kNValidate, 0, s>>>(L.rows, L.red_blocks, spec, L.red_out);
   XAC_CUDA(cudaGetLastError());
   XAC_CUDA(cudaMemcpyAsync(L.host_out, L.red_out, kNValidate * sizeof(double), cudaMemcpyDeviceToHost, s));
+  XAC_CUDA(L.copy_status(s));
   XAC_CUDA(cudaStreamSynchronize(s));
   std::memcpy(out_host, L.host_out, kNValidate * sizeof(double));
-  return XAC_OK;
+  return L.read_status("xac_lattice_validate");
 }
 
 int xac_lattice_state_bytes(const xac_lattice* lat, size_t* bytes) {
@@ -1260,8 +1288,9 @@ int xac_lattice_save_state(xac_lattice* lat, void* host_dst, size_t bytes, void*
   const float* f[5] = {L.rho, L.ux, L.uy, L.uz, L.T};
   for (int k = 0; k < 5; ++k)
     XAC_CUDA(cudaMemcpyAsync(dst + 64 + pb + qb + k * nf, f[k], nf, cudaMemcpyDeviceToHost, s));
+  XAC_CUDA(L.copy_status(s));
   XAC_CUDA(cudaStreamSynchronize(s));
-  return XAC_OK;
+  return L.read_status("xac_lattice_save_state");
 }
 
 int xac_lattice_load_state(xac_lattice* lat, const void* host_src, size_t bytes, void* stream) {
@@ -1293,7 +1322,7 @@ int xac_lattice_load_state(xac_lattice* lat, const void* host_src, size_t bytes,
   set_scalar_kernel<<<1, 1, 0, s>>>(L.u_in, u_in);
   XAC_CUDA(cudaMemsetAsync(L.status, 0, sizeof(unsigned), s));
   XAC_CUDA(cudaStreamSynchronize(s));
-  L.failed = false;
+  L.failed = L.unread = false;
   L.cur = 0;
   L.step = hdr[5];
   L.own_pending = hdr[6] != 0;
@@ -1434,8 +1463,10 @@ int xac_lattice_run(xac_lattice* lat, const xac_run_opts* o, xac_run_result* res
       c.dQ = dQ;
       c.u_in = L.u_in_host;
       XAC_CUDA(cudaMemcpyAsync(L.run_ctl, &c, sizeof(RunCtl), cudaMemcpyHostToDevice, s));
+      if (L.staged()) XAC_CUDA(L.note_staged(s));
       XAC_CUDA(cudaGraphLaunch(ex, s));
       XAC_CUDA(cudaMemcpyAsync(&c, L.run_ctl, sizeof(RunCtl), cudaMemcpyDeviceToHost, s));
+      XAC_CUDA(L.copy_status(s));
       XAC_CUDA(cudaStreamSynchronize(s));
       L.step += c.step - step;
       L.macro_step = L.step;
@@ -1449,16 +1480,8 @@ int xac_lattice_run(xac_lattice* lat, const xac_run_opts* o, xac_run_result* res
       dT = c.dT;
       dQ = c.dQ;
       std::memcpy(res->last_stats, c.last, sizeof(c.last));
-      if (L.staged()) {  // the staged kernel's bounded wait reports here
-        unsigned stw = 0;
-        XAC_CUDA(cudaMemcpy(&stw, L.status, sizeof(stw), cudaMemcpyDeviceToHost));
-        if (stw) {
-          L.failed = true;
-          set_error("xac_lattice_run: a staged step kernel gave up waiting for its copies (status %u); the lattice "
-                    "refuses further work until init_fields or load_state", stw);
-          return XAC_ETIMEOUT;
-        }
-      }
+      r = L.read_status("xac_lattice_run");
+      if (r != XAC_OK) return r;
       if (c.diverged) {
         diverged = 1;
         break;
