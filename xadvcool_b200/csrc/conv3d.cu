@@ -869,13 +869,46 @@ __global__ void __launch_bounds__(256) bias_grad_partial_kernel(const __nv_bfloa
   }
 }
 
+// dw[tap][co][ci] over the voxels u of the input, d_out[u - off(tap)] a zero outside the volume; the caller's segment takes
+// its eighth of them. Products are exact in FP64; a sum that is NaN stays one and ends.
+__device__ __noinline__ double wgrad_direct(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout,
+                                            const ConvShape& s, long long e, int seg) {
+  const int ci = (int)(e % s.Ci), co = (int)(e / s.Ci % s.Co), tap = (int)(e / s.Ci / s.Co), nd = s.ksize, kr = nd >> 1;
+  const int dz = tap / (nd * nd) - kr, dy = tap / nd % nd - kr, dx = tap % nd - kr;
+  const long long V = (long long)s.N * s.D * s.H * s.W, end = V * (seg + 1) / 8;
+  long long u = V * seg / 8;
+  int x = (int)(u % s.W), y = (int)(u / s.W % s.H), z = (int)(u / s.W / s.H % s.D);
+  const long long off = ((long long)dz * s.H + dy) * s.W + dx;
+  double t = 0.0;
+  for (; u < end && t == t; ++u) {
+    const bool inside = (unsigned)(z - dz) < (unsigned)s.D && (unsigned)(y - dy) < (unsigned)s.H &&
+                        (unsigned)(x - dx) < (unsigned)s.W;
+    const float d = inside ? __bfloat162float(dout[(u - off) * s.Co + co]) : 0.0f;
+    t += (double)d * (double)__bfloat162float(in[u * s.Ci + ci]);
+    if (++x == s.W) {
+      x = 0;
+      if (++y == s.H) {
+        y = 0;
+        if (++z == s.D) z = 0;
+      }
+    }
+  }
+  return t;
+}
+
 // The partial sums of both, one launch. dw[e] = sum of the CTAs' partials: a block sums 32 values, 8 segments of the CTAs
 // each in order, then the segments in order. The blocks after those take db: a warp per channel, 32 strided sums
 // of the bias partials, then a fixed tree.
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, int n, long long count,
+// The tiles multiply d_out by the zeros around the input and the input by the zeros around d_out, and an infinity times
+// those is a NaN in taps that do not use the voxel. Such a sum is never finite, so a value that is not is summed anew.
+__global__ void __launch_bounds__(256, 8) wgrad_reduce_kernel(const float* __restrict__ partial, int n, long long count,
                                                            float* __restrict__ dw, const float* __restrict__ bias_partial,
-                                                           int bias_rows, int Co, float* __restrict__ db) {
+                                                           int bias_rows, const __nv_bfloat16* __restrict__ in,
+                                                           const __nv_bfloat16* __restrict__ dout,
+                                                           const __grid_constant__ ConvShape s,
+                                                           float* __restrict__ db) {
   __shared__ float part[8][33];
+  const int Co = s.Co;
   const int x = threadIdx.x & 31, seg = threadIdx.x >> 5;
   const long long dw_blocks = (count + 31) / 32;
   if (blockIdx.x >= dw_blocks) {
@@ -897,9 +930,23 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
   }
   part[seg][x] = t;
   __syncthreads();
+  bool finite = true;
   if (seg == 0 && e < count) {
     for (int k = 1; k < 8; ++k) t += part[k][x];
     dw[e] = t;
+    finite = isfinite(t);
+  }
+  if (__syncthreads_and(finite)) return;
+  __shared__ double direct[8][33];
+  __shared__ int redo[32];
+  if (seg == 0) redo[x] = !finite;
+  __syncthreads();
+  if (redo[x]) direct[seg][x] = wgrad_direct(in, dout, s, e, seg);
+  __syncthreads();
+  if (!finite) {
+    double sum = 0.0;
+    for (int k = 0; k < 8; ++k) sum += direct[k][x];
+    dw[e] = (float)sum;
   }
 }
 
@@ -1273,7 +1320,7 @@ int xac_conv3d_weight_grad(const void* in, int N, int D, int H, int W, int Ci, c
   if (db)
     bias_grad_partial_kernel<<<rows, 256, 0, st>>>((const __nv_bfloat16*)dout, V, Co, bias_partial);
   wgrad_reduce_kernel<<<(unsigned)((count + 31) / 32) + (db ? (Co + 7) / 8 : 0), 256, 0, st>>>(
-      partial, pl.ctas, count, dw, bias_partial, rows, Co, db);
+      partial, pl.ctas, count, dw, bias_partial, rows, (const __nv_bfloat16*)in, (const __nv_bfloat16*)dout, s, db);
   XAC_CUDA(cudaGetLastError());
   return XAC_OK;
 }
