@@ -190,13 +190,13 @@ __global__ void __launch_bounds__(256) pattern_copy_kernel(const SP* __restrict_
   const bool fill_q = (__ballot_sync(0xffffffffu, valid) & sector_group<SQ>(lane)) != 0u;
   const uint32_t e0 = pop_base(r, x, g, RL);
   if (fluid) {
-    const FluidAt<SP> P = fluid_at(Pin, r, x, g, ftab);
+    const auto P = fluid_at(Pin, r, x, g, ftab);
 #define XAC_PC_P(I) Pout[P.own_index(I)] = ((lw >> (I)) & 1u) ? __ldg(P.own(opp_of(I))) : __ldg(P.template pull<I>());
     XAC_FOR19(XAC_PC_P)
 #undef XAC_PC_P
   }
   if (valid) {
-    const Rows<SQ, kT> Q = rows_at<kT>(Qin, e0, g, RL);
+    const auto Q = rows_at<kT>(Qin, e0, g, RL);
 #define XAC_PC_Q(I) Qout[e0 + (I) * RL] = __ldg(Q.template pull<I>());
     XAC_FOR19(XAC_PC_Q)
 #undef XAC_PC_Q
@@ -317,6 +317,15 @@ static_assert(kStatusSlot >= kNStats && kStatusSlot >= kNMetrics && kStatusSlot 
 
 struct LatticeImpl {
   Geom g{};
+  SlotTables tables() const {
+    SlotTables t;
+    for (int i = 0; i < kQ; ++i) {
+      t.run[i] = (uint32_t)((long long)i * g.ns);
+      t.own_off[i] = (uint32_t)(i * g.pitch);
+      t.pull_off[i] = (uint32_t)((i - ey_of(i) * kQ) * g.pitch - ex_of(i));
+    }
+    return t;
+  }
   int precision = XAC_FP32;
   size_t p_elem = 4, q_elem = 4;  // bytes per fluid / thermal population
   double tau_fluid = 0.6, Pr = 7.0, k_ratio = 628.0, u_inlet_nominal = 0.03, rho_outlet = 1.0, t_inlet = 25.0,
@@ -490,6 +499,7 @@ struct LatticeImpl {
     float* const field[3] = {ux, uy, uz};
     auto uset = [&](int back, int k) { return u_step + ((size_t)(back % kUSets) * 3 + k) * g.ncell; };
     a.p = params();
+    a.tab = tables();
     a.link = link;
     a.qsrc = qsrc;
     a.u_in = u_in;
@@ -858,7 +868,6 @@ std::vector<uint2> fluid_table(const uint8_t* type, Geom& g, uint32_t* nonsolid,
   g.ns = ((long long)k + 31) / 32 * 32;
   if (g.ns == 0) g.ns = 32;
   g.np = (long long)kQ * g.ns;
-  for (int i = 0; i < kQ; ++i) g.run[i] = (uint32_t)((long long)i * g.ns);
   return tab;
 }
 
@@ -911,10 +920,6 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   L.g.rows = ny * nz;
   L.g.guard = (long long)(ny + 2) * kQ * L.g.pitch;
   L.g.N = (long long)L.g.rows * kQ * L.g.pitch + 2 * L.g.guard;
-  for (int i = 0; i < kQ; ++i) {
-    L.g.own_off[i] = (uint32_t)(i * L.g.pitch);
-    L.g.pull_off[i] = (uint32_t)((i - ey_of(i) * kQ) * L.g.pitch - ex_of(i));
-  }
   L.precision = d->precision;
   L.p_elem = (d->precision == XAC_FP32 || d->precision == XAC_FP32_T16) ? 4 : 2;
   L.q_elem = d->precision == XAC_FP32 ? 4 : 2;

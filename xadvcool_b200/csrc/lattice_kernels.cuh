@@ -68,7 +68,13 @@ struct Geom {
   int nt;           // 32-cell words of a row: pitch / 32
   long long ns;     // slots of a fluid population run: the non-solid cells, rounded up to a multiple of 32
   long long np;     // elements of one fluid population array: 19*ns
-  uint32_t run[kQ];  // start of each direction's run: i*ns
+};
+
+// Offsets of the populations by direction, for kernels that take them as parameters (constant operands of the index
+// additions) instead of working them out. Only the split step does (kTab): 228 bytes of parameters cost every launch of a
+// small lattice's step, and in the batch kernel they are loads from shared memory where the arithmetic is free.
+struct SlotTables {
+  uint32_t run[kQ];  // start of each direction's fluid run: i*ns
   // thermal populations: own value of direction i (i*pitch); its source ((i - e_y*19)*pitch - e_x) from the row one z-slab
   // against e_z
   uint32_t own_off[kQ], pull_off[kQ];
@@ -167,7 +173,7 @@ struct StepParams {
 // in the rows one z-slab below (source of directions with ez = +1) and above (ez = -1). own(i) is the cell's
 // direction i, pull<I>() the source of direction I (a compile-time offset from one of the three pointers when
 // kT > 0).
-template <typename S, int kT>
+template <typename S, int kT, bool kTab>
 struct Rows {
   const S* c;
   const S* zm;
@@ -182,27 +188,31 @@ struct Rows {
   }
 };
 // Runtime row length: one base pointer and 32-bit element indices (every index of a population array fits in 31
-// bits); the offsets are kernel parameters, constant operands of the index additions.
-template <typename S>
-struct Rows<S, 0> {
+// bits), so an address is formed right before its load instead of 19 64-bit pointers living at once.
+template <typename S, bool kTab>
+struct Rows<S, 0, kTab> {
   const S* base;
   uint32_t c, zm, zp;
-  const Geom* g;
-  __device__ __forceinline__ const S* own(int i) const { return base + (c + g->own_off[i]); }
+  int RL;
+  const SlotTables* tab;
+  __device__ __forceinline__ const S* own(int i) const {
+    return base + (c + (kTab ? tab->own_off[i] : (uint32_t)(i * RL)));
+  }
   template <int I>
   __device__ __forceinline__ const S* pull() const {
     const uint32_t b = ez_of(I) > 0 ? zm : (ez_of(I) < 0 ? zp : c);
-    return base + (b + g->pull_off[I]);
+    return base + (b + (kTab ? tab->pull_off[I] : (uint32_t)((I - ey_of(I) * kQ) * RL - ex_of(I))));
   }
 };
-template <int kT, typename S>
-__device__ __forceinline__ Rows<S, kT> rows_at(const S* base, uint32_t e0, const Geom& g, int pitch) {
+template <int kT, bool kTab = false, typename S>
+__device__ __forceinline__ Rows<S, kT, kTab> rows_at(const S* base, uint32_t e0, const Geom& g, int pitch,
+                                                     const SlotTables* tab = nullptr) {
   if constexpr (kT > 0) {
     const long long slab = (long long)g.ny * kQ * pitch;
     return {base + e0, base + e0 - slab, base + e0 + slab, pitch};
   } else {
     const uint32_t slab = (uint32_t)g.ny * kQ * (uint32_t)pitch;
-    return {base, e0, e0 - slab, e0 + slab, &g};
+    return {base, e0, e0 - slab, e0 + slab, pitch, tab};
   }
 }
 
@@ -224,13 +234,13 @@ __host__ __device__ constexpr int fluid_row_ez(int j) { return j == 2 || j == 4 
 // own(opp)). rk[j] is the number of non-solid cells before the cell's x in row slot j; the source of a
 // direction with e_x = 0 is that cell, with e_x = +1 the one before it (x-1 is non-solid), with e_x = -1 the next
 // one (x+1), which is one further when x itself is non-solid in that row (bit j of nb).
-template <typename S>
+template <typename S, bool kTab>
 struct FluidAt {
   const S* base;
-  const uint32_t* run;  // run[i] = i*ns (kernel parameters: a constant operand of the index additions)
-  uint32_t k, nb;
+  const uint32_t* run;  // run[i] = i*ns, with kTab
+  uint32_t ns, k, nb;
   uint32_t rk[8];
-  __device__ __forceinline__ uint32_t own_index(int i) const { return k + run[i]; }
+  __device__ __forceinline__ uint32_t own_index(int i) const { return k + (kTab ? run[i] : (uint32_t)i * ns); }
   __device__ __forceinline__ const S* own(int i) const { return base + own_index(i); }
   template <int I>
   __device__ __forceinline__ uint32_t pull_index() const {
@@ -243,7 +253,7 @@ struct FluidAt {
       if constexpr (ex_of(I) == 1) s -= 1u;
       if constexpr (ex_of(I) == -1) s += (nb >> j) & 1u;
     }
-    return s + run[I];
+    return s + (kTab ? run[I] : (uint32_t)I * ns);
   }
   template <int I>
   __device__ __forceinline__ const S* pull() const {
@@ -255,12 +265,14 @@ __host__ __device__ __forceinline__ uint32_t ftab_index(const Geom& g, uint32_t 
   return (r + (uint32_t)g.ny + 1u) * (uint32_t)g.nt + (x >> 5);
 }
 // the view of the non-solid cell in slot k, bit `bit` of table entry t0
-template <typename S>
-__device__ __forceinline__ FluidAt<S> fluid_at_entry(const S* base, uint32_t k, uint32_t t0, uint32_t bit, const Geom& g,
-                                                     const uint2* __restrict__ ftab) {
-  FluidAt<S> a;
+template <bool kTab, typename S>
+__device__ __forceinline__ FluidAt<S, kTab> fluid_at_entry(const S* base, uint32_t k, uint32_t t0, uint32_t bit,
+                                                           const Geom& g, const uint2* __restrict__ ftab,
+                                                           const uint32_t* run) {
+  FluidAt<S, kTab> a;
   a.base = base;
-  a.run = g.run;
+  a.run = run;
+  a.ns = (uint32_t)g.ns;
   a.k = k;
   const uint32_t below = (1u << bit) - 1u;
   a.nb = 0u;
@@ -275,11 +287,11 @@ __device__ __forceinline__ FluidAt<S> fluid_at_entry(const S* base, uint32_t k, 
 }
 // the view of cell (row r, x), which must be non-solid; the nine table loads are the same for a whole warp
 template <typename S>
-__device__ __forceinline__ FluidAt<S> fluid_at(const S* base, uint32_t r, uint32_t x, const Geom& g,
+__device__ __forceinline__ FluidAt<S, false> fluid_at(const S* base, uint32_t r, uint32_t x, const Geom& g,
                                                const uint2* __restrict__ ftab) {
   const uint32_t t0 = ftab_index(g, r, x), bit = x & 31u;
   const uint2 e = __ldg(ftab + t0);
-  return fluid_at_entry(base, e.y + (uint32_t)__popc(e.x & ((1u << bit) - 1u)), t0, bit, g, ftab);
+  return fluid_at_entry<false>(base, e.y + (uint32_t)__popc(e.x & ((1u << bit) - 1u)), t0, bit, g, ftab, nullptr);
 }
 
 // the nine pairs of opposite directions
@@ -503,11 +515,12 @@ __device__ __forceinline__ void thermal_gather(const Acc& Q, const StepParams& p
 
 // Temperature and collision of any cell, with the cell's fluid velocity u (0 in solids; kRest: 0 in every lane of the warp;
 // kHeat false: no lane of the warp is heated)
-template <typename S, bool kOwn, int kLd, int kT, bool kRest = false, bool kHeat = true>
+template <typename S, bool kOwn, int kLd, int kT, bool kTab = false, bool kRest = false, bool kHeat = true>
 __device__ __forceinline__ void thermal_collide(const uint32_t c, S* __restrict__ Qo, const float* __restrict__ qsrc,
                                                 const float* __restrict__ T0, const StepParams& p, const uint32_t lw,
-                                                const float (&G)[kQ], const float ux, const float uy,
-                                                const float uz) {
+                                                const float (&G)[kQ], const float ux, const float uy, const float uz,
+                                                const SlotTables* tab = nullptr) {
+  const int RL = row_len<kT>(p.g);
   const int type = link_type(lw);
   const float Tb = p.T_ref;
   float T;
@@ -529,7 +542,7 @@ __device__ __forceinline__ void thermal_collide(const uint32_t c, S* __restrict_
   {                                                                              \
     float v = G[I] - omega_t * (G[I] - (GE));                                    \
     if (heated && q > 0.0f) v += (w_of(I) * srcf) * q;                           \
-    Pop<S>::st(Qo + (kT > 0 ? (uint32_t)((I) * kT) : p.g.own_off[I]), v, w_of(I) * Tb); \
+    Pop<S>::st(Qo + (kT == 0 && kTab ? tab->own_off[I] : (uint32_t)((I) * RL)), v, w_of(I) * Tb); \
   }
   if (kRest) {  // u = 0: every bracket of the equilibrium is exactly 1
 #define XAC_TREST(I) XAC_TOUT(I, w_of(I) * T)
@@ -575,7 +588,7 @@ __device__ __forceinline__ void coupled_cell(const uint32_t c, const uint32_t r,
   const bool fluid = valid && link_type(lw) != kSolid;
   float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
   if (fluid) {
-    const FluidAt<SP> P = fluid_at(Pin, r, x, p.g, p.ftab);
+    const auto P = fluid_at(Pin, r, x, p.g, p.ftab);
     fluid_cell<SP, kMacro, kLd>(c, P, Pout, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, rho, ux, uy, uz);
   } else if (valid) {
     solid_cell<kMacro>(c, rho_o, ux_o, uy_o, uz_o);
@@ -630,6 +643,7 @@ struct SplitArgs {
   uint32_t frev, trev;          // blocks in reverse order
   int own;                      // the thermal step reads its populations unstreamed (first step)
   StepParams p;
+  SlotTables tab;
 };
 
 constexpr int kCellXShift = 24;
@@ -649,15 +663,15 @@ __device__ __forceinline__ void split_fluid(const SplitArgs& a, const uint32_t k
   const uint2 info = __ldg(a.cells + k);
   const uint32_t lw = info.x & ~kCellXMask, x31 = (info.x & kCellXMask) >> kCellXShift;
   if (!kEnd && link_type(lw) != kFluid) return;
-  FluidAt<SP> P;
+  FluidAt<SP, true> P;
   float F[kQ];
   if (kEnd) {
     P.base = (const SP*)a.Pin;
-    P.run = a.p.g.run;
+    P.run = a.tab.run;
     P.k = k;
     fluid_gather_end<SP, 0>(P, a.u_in, a.p, lw, F);
   } else {
-    P = fluid_at_entry<SP>((const SP*)a.Pin, k, info.y, x31, a.p.g, a.p.ftab);
+    P = fluid_at_entry<true>((const SP*)a.Pin, k, info.y, x31, a.p.g, a.p.ftab, a.tab.run);
     fluid_gather<SP, 0>(P, lw, F);
   }
   float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
@@ -688,7 +702,7 @@ __device__ __forceinline__ void split_thermal(const SplitArgs& a, const uint32_t
   const bool fluid = link_type(lw) != kSolid;
   const bool moving = __any_sync(0xffffffffu, fluid), heated = __any_sync(0xffffffffu, (lw & kHeatedBit) != 0u);
   if (valid) {
-    const Rows<SQ, kT> Q = rows_at<kT>((const SQ*)a.Qin, e0, g, RL);
+    const auto Q = rows_at<kT, true>((const SQ*)a.Qin, e0, g, RL, &a.tab);
     SQ* Qo = (SQ*)a.Qout + e0;
     // the populations are on their way while the cell's slot and then its velocity are looked up
     const uint2 e = __ldg(a.p.ftab + ftab_index(g, r, x));
@@ -702,10 +716,11 @@ __device__ __forceinline__ void split_thermal(const SplitArgs& a, const uint32_t
       uy = __ldg(a.ui[1] + k);
       uz = __ldg(a.ui[2] + k);
     }
-    if (!kPlain && a.own) thermal_collide<SQ, true, 0, kT>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
-    else if (heated) thermal_collide<SQ, false, 0, kT>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
-    else if (moving) thermal_collide<SQ, false, 0, kT, false, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
-    else thermal_collide<SQ, false, 0, kT, true, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz);
+    if (!kPlain && a.own) thermal_collide<SQ, true, 0, kT, true>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz, &a.tab);
+    else if (heated) thermal_collide<SQ, false, 0, kT, true>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz, &a.tab);
+    else if (moving)
+      thermal_collide<SQ, false, 0, kT, true, false, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz, &a.tab);
+    else thermal_collide<SQ, false, 0, kT, true, true, false>(c, Qo, a.qsrc, a.T0, a.p, lw, G, ux, uy, uz, &a.tab);
     if (!kPlain && a.solid[0] && !fluid) solid_cell<true>(c, a.solid[0], a.solid[1], a.solid[2], a.solid[3]);
   }
   pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, (SQ*)a.Qout, e0, g);
@@ -812,7 +827,7 @@ __global__ void __launch_bounds__(kT) coupled_qstage_kernel(const SP* __restrict
   const uint32_t e0 = pop_base(r, x, p.g, kT);
   float rho, ux = 0.0f, uy = 0.0f, uz = 0.0f;
   if (valid && link_type(lw) != kSolid) {
-    const FluidAt<SP> P = fluid_at(Pin, r, x, p.g, p.ftab);
+    const auto P = fluid_at(Pin, r, x, p.g, p.ftab);
     fluid_cell<SP, kMacro, 0>(c, P, Pout, u_in_ptr, rho_o, ux_o, uy_o, uz_o, p, lw, rho, ux, uy, uz);
   } else if (valid) {
     solid_cell<kMacro>(c, rho_o, ux_o, uy_o, uz_o);
@@ -871,7 +886,7 @@ __device__ __forceinline__ float finalize_T_cell(const S* __restrict__ Qin, cons
   const float Tb = p.T_ref;
   const int RL = p.g.pitch;
   const uint32_t r = c / (uint32_t)p.g.nx, x = c - r * (uint32_t)p.g.nx;
-  const Rows<S, 0> Q = rows_at<0>(Qin, pop_base(r, x, p.g, RL), p.g, RL);
+  const auto Q = rows_at<0>(Qin, pop_base(r, x, p.g, RL), p.g, RL);
   float T = 0.0f;
   if (type == kInlet) {
 #pragma unroll
