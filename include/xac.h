@@ -343,7 +343,7 @@ int xac_conv3d_weight_grad(const void *in, int N, int D, int H, int W, int Ci, c
                            float *partial, float *dw, float *db, void *stream);
 int xac_conv3d_partial_floats(int N, int D, int H, int W, int Ci, int Co, int ksize, long long *count);
 /* Reads and clears the device-side status of the convolution kernels (synchronises the device): bit 0 set means a
- * bounded wait inside a tensor-core kernel ran out, and that launch left its output unwritten. */
+ * bounded wait inside a tensor-core kernel ran out, and that launch left its output incomplete: discard it. */
 int xac_conv3d_status(int *flags);
 /* out = GELU(gamma h + beta), h = (y - mean) rstd, mean and rstd [N][G] over V voxels and C/G channels; BF16 [N][V][C]
  * in and out, FP32 between, every operation rounded by itself. C a power of two (8..256), C/G a multiple of 4, volumes

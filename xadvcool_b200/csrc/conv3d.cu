@@ -412,9 +412,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
         }
         u += nz;
       }
-      // an abort may leave copies that no role waited for: let them land before the block's memory goes back
-      if (*abort_v)
-        for (int k = seq > pl.NS ? seq - pl.NS : 0; k < seq; ++k) mbar_wait(bar.afull(k % pl.NS), (k / pl.NS) & 1);
+      // an abort may leave copies that no role waits for: each lands before the block's memory goes back
+      for (int k = seq > pl.NS ? seq - pl.NS : 0; k < seq; ++k) mbar_wait(bar.afull(k % pl.NS), (k / pl.NS) & 1);
     }
   } else if (warp == kEpiWarps + kMmaWarps + 1) {
     // ---- weights: all of them at once, or the stages of one unit again and again (with the unit's slice of Co)
@@ -423,7 +422,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
         mbar_expect_tx(bar.bfull(0), (uint32_t)(taps * nkc) * bblk_bytes);
         for (int k = 0; k < nkc; ++k)
           tma_load_3d(b0 + (uint32_t)(k * taps) * bblk_bytes, &tw, k * pl.KB, 0, 0, bar.bfull(0));
-        if (*abort_v) mbar_wait(bar.bfull(0), 0);
+        mbar_wait(bar.bfull(0), 0);
       } else {
         int st = 0;
         long long seq = 0;
@@ -448,9 +447,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
               }
             }
         }
-        if (*abort_v)
-          for (long long k = seq > pl.bs ? seq - pl.bs : 0; k < seq; ++k)
-            mbar_wait(bar.bfull((int)(k % pl.bs)), (uint32_t)(k / pl.bs) & 1u);
+        for (long long k = seq > pl.bs ? seq - pl.bs : 0; k < seq; ++k)
+          mbar_wait(bar.bfull((int)(k % pl.bs)), (uint32_t)(k / pl.bs) & 1u);
       }
     }
   } else if (warp >= kEpiWarps) {
@@ -525,9 +523,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
       mbar_arrive(bar.cempty(buf));
     }
   }
-  // every MMA issued has finished before the tensor memory goes back
+  // Every MMA issued has finished before the tensor memory goes back. Only the warps that issue them wait on done, so its
+  // limit counts from the end of their own work; the others stand at the barrier, where a long launch is no failure.
   __syncwarp();
-  mbar_wait(bar.done(), 0);
+  if (warp >= kEpiWarps && warp < kEpiWarps + nmw) mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
@@ -716,11 +715,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_wgrad_kernel(const __grid_
         }
         u += nz;
       }
-      // an abort may leave copies that no role waited for: let them land before the block's memory goes back
-      if (*abort_v) {
-        for (int k = xseq > pl.NX ? xseq - pl.NX : 0; k < xseq; ++k) mbar_wait(bar.xfull(k % pl.NX), (k / pl.NX) & 1);
-        for (int k = dseq > 2 ? dseq - 2 : 0; k < dseq; ++k) mbar_wait(bar.dfull(k & 1), (k >> 1) & 1);
-      }
+      // as in the forward kernel: each copy lands before the block's memory goes back
+      for (int k = xseq > pl.NX ? xseq - pl.NX : 0; k < xseq; ++k) mbar_wait(bar.xfull(k % pl.NX), (k / pl.NX) & 1);
+      for (int k = dseq > 2 ? dseq - 2 : 0; k < dseq; ++k) mbar_wait(bar.dfull(k & 1), (k >> 1) & 1);
     }
   } else if (warp >= kWgEpiWarps) {
     const int t0 = warp - kWgEpiWarps;
@@ -829,7 +826,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_wgrad_kernel(const __grid_
     }
   }
   __syncwarp();
-  mbar_wait(bar.done(), 0);
+  if (warp >= kWgEpiWarps && warp < kWgEpiWarps + nmw) mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
