@@ -230,14 +230,15 @@ int xac_lattice_fields(xac_lattice *lat, float *rho, float *u, float *T, void *s
 int xac_lattice_set_inlet(xac_lattice *lat, double u_inlet, void *stream);
 int xac_lattice_get_inlet(xac_lattice *lat, double *u_inlet, void *stream);
 int xac_lattice_steps_done(const xac_lattice *lat, long long *steps);
-/* Launch shape of the step: threads per block (64, 128, 256) and the variant: 0 = the fluid and the thermal lattice in
- * kernels of their own, the fluid a step ahead; 1 = one block per row for both, its thermal input staged in shared
- * memory by bulk copies while the fluid lattice runs (row lengths up to 320; longer ones run variant 0). A lattice
- * starts with block 64 and the variant its size, storage and mask suggest. Variant 1 waits for its copies with a bounded
+/* Launch shape of the step: threads per block (64, 128, 256) and the variant: 0 = one thread per row position for both
+ * lattices, or the two lattices in kernels of their own, the fluid a step ahead (by size, storage, mask and length of the
+ * run); 1 = one block per row for both, its thermal input staged in shared memory by bulk copies while the fluid lattice
+ * runs (row lengths up to 320; longer ones run variant 0). A lattice
+ * starts with the shape its size, storage and mask suggest. Variant 1 waits for its copies with a bounded
  * wait; if a wait ever gives up, the next call that hands results to the caller (stats, run, fields, scalars, validate,
  * save-state) returns XAC_ETIMEOUT, also after a change of variant, and the lattice refuses every further call of those and
- * step with XAC_ETIMEOUT until xac_lattice_init_fields or xac_lattice_load_state rewrites its populations. Results do not depend on the shape (every cell runs the same
- * arithmetic); xadvcool_b200.autotune picks it. */
+ * step with XAC_ETIMEOUT until xac_lattice_init_fields or xac_lattice_load_state rewrites its populations. Results do not
+ * depend on the shape (every cell runs the same arithmetic); xadvcool_b200.autotune picks it. */
 int xac_lattice_tune(xac_lattice *lat, int block, int variant);
 int xac_lattice_get_tune(const xac_lattice *lat, int *block, int *variant);
 /* Diagnostic, no reference counterpart: the floor that the fused step's memory access pattern sets for this
@@ -250,6 +251,9 @@ int xac_lattice_pattern_copy(xac_lattice *lat, int launches, double *us_per_laun
 /* Test hook: writes the lattice's step status word as a staged step kernel whose wait gave up would (no kernel
  * runs), so that a test sees the lattice refuse work and recover after xac_lattice_init_fields. */
 int xac_test_set_step_status(xac_lattice *lat, unsigned value, void *stream);
+/* Test hook: runs of any length take the one-pass (0), the split (1) or the staged step (2; rows up to 320), whatever the
+ * lattice's size suggests; -1 goes back to that. */
+int xac_test_step_form(xac_lattice *lat, int form);
 /* Inputs of generate_dataset.py:80 compute_macroscopic_metrics that are not fields. */
 typedef struct xac_scalar_params {
     int buf;            /* inlet/outlet buffer length along x (10, generate_dataset.py:90)            */

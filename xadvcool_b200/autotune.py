@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 BLOCKS = (64, 128, 256)
-VARIANTS = (0, 1)  # 0: the two lattices in kernels of their own; 1: thermal rows staged in shared memory (block = row)
+VARIANTS = (0, 1)  # 0: one-pass or split step; 1: thermal rows staged in shared memory (block = row)
 
 
 def _cache_path() -> Path:

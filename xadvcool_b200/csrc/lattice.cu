@@ -333,18 +333,60 @@ struct LatticeImpl {
   float tau_th_f = 0.5f, tau_th_s = 0.5f;
   float relax[5] = {1.0f, 1.0f, 1.0f, 0.5f, 0.5f};  // omega_f, omega_tf, omega_ts, srcf_f, srcf_s (device-computed)
   float u_in_host = 0.0f;
-  int tune_block = 64;   // threads per block of the split step's kernels (128: +1 to +4%, 256: +8 to +12%)
-  int tune_variant = 0;  // 0: split step, the two lattices in kernels of their own; 1: thermal rows staged in shared memory
-  // The launch shape a lattice starts with. The staged step is one launch where the split step takes two, and wins where
-  // launches decide: at 98k row positions 5.7 against 6.6 us in FP32 and 5.9 against 6.8 in FP16; at 197k it is 9.5 against
-  // 9.0 and 10.0 against 9.2, at 655k 27.6 against 27.1 and 26.0 against 20.5. (Its one-warp blocks at row length 32 pay
-  // off in 16 bits only: 30x20x12 4.9 against 4.3 us in FP32, 5.2 against 5.8 in FP16.) In FP32, where memory decides, it
-  // also wins where rows are all fluid or all solid and the split step has no idle lanes to save: straight channels
-  // 148x128x32 26.8 against 27.5 us, 301x203x61 148 against 159; at 60% full warps (pins) 24.3 against 23.2.
-  void default_tune(double full_lanes) {
-    const bool small = (long long)g.rows * g.pitch <= 131072;
-    const bool staged = small ? g.pitch >= 64 || precision != XAC_FP32 : precision == XAC_FP32 && full_lanes >= 0.8;
-    tune_variant = staged && g.pitch <= kMaxStagedRow ? 1 : 0;
+  int tune_block = 128;  // threads per block of the one-pass step and of the split step's kernels
+  int tune_variant = 0;  // 0: one-pass or split step, by form(); 1: thermal rows staged in shared memory
+  double share = 1.0, lanes = 1.0;  // non-solid cells, of all cells and of the lanes of warps that hold one
+  long long positions() const { return (long long)g.rows * g.pitch; }
+  static constexpr long long kSmall = 131072, kMid = 327680, kHalfM = 1 << 19, k1M = 1 << 20, k2M = 1 << 21;
+
+  // The three forms of a step; all give the same bits. Below, us a step in runs of 100, at row positions and share of
+  // non-solid cells; FP16 stands for BF16 too, whose times are within 2%.
+  enum class Form { kRow, kSplit, kStaged };
+  // Variant 0, runs of 8 steps and more: split or one-pass. Two launches do not pay on a small lattice (33k 5.2 against
+  // 4.4 in FP32, 5.9 against 5.2 in FP16; 110k 7.1 against 5.9 and 6.9 against 6.8). In FP32 memory decides, and the split
+  // step's full warps buy less than its detour of u costs, except where most lanes of a one-pass warp are idle: lanes 0.32
+  // at 655k 23.0 against 24.2, 0.27 at 1.15M 35.9 against 40.5, but 0.49 at 655k 28.1 against 27.4; large lattices gain
+  // earlier, 0.47 at 3.96M 161 against 167, 0.48 at 1.38M without a staged form 51.8 against 52.6. In 16 bits issue
+  // decides: share 0.55 at 655k 21.7 against 26.4, at 3.96M 132 against 159; with few solids few lanes are idle: share
+  // 0.70 at 295k 14.4 against 13.1, but 0.74 at 491k 19.7 against 20.9; rows of 340 at share 0.72 57.9 against 54.5. FP32
+  // fluid with FP16 thermal: 0.55 at 655k 23.4 against 26.9; rows of 340 at 0.14 38.1 against 46.3, at 0.41 49.6 against
+  // 47.0.
+  bool split_pays() const {
+    const long long p = positions();
+    const bool stageable = g.pitch <= kMaxStagedRow;
+    if (p <= kSmall) return false;
+    if (precision == XAC_FP32) return lanes < (p > k2M || (p > k1M && !stageable) ? 0.5 : 0.4);
+    if (precision == XAC_FP32_T16) return share < (stageable ? 0.62 : 0.3);
+    return share < 0.62 || (stageable && p > kMid);
+  }
+  // Shorter runs are launched one kernel after the other, where the split step's two halves do not overlap: 655k FP32 36.4
+  // against 30.6 us a step in runs of 7, FP16 32.3 against 28.9. It keeps 16-bit lattices that are large (3.96M 148 against
+  // 163) or hollow (share 0.2 at 655k 25.0 against 27.3).
+  int forced = -1;  // a test's choice of the form
+  Form form(int n) const {
+    if (forced >= 0) return (Form)forced;
+    if (tune_variant == 1 && g.pitch <= kMaxStagedRow) return Form::kStaged;
+    if (!split_pays()) return Form::kRow;
+    if (n >= 8) return Form::kSplit;
+    const long long p = positions();
+    return precision != XAC_FP32 && (p > k2M || (share < 0.3 && p > kHalfM)) ? Form::kSplit : Form::kRow;
+  }
+  bool staged() const { return form(1) == Form::kStaged; }
+  // The launch shape a lattice starts with: staged where that is the fastest of the three. FP32: 1.15M 41.4, 46.0 and 51.0
+  // against 43.4, 47.0 and 51.0 (one-pass), 3.96M 147 and 165 against 153 and 169, but at 655k 26.9 and 29.0 against 26.2
+  // and 28.2. FP16: 33k 4.6 against 5.2, 110k 6.6 against 6.8; at 197k 9.5 against 8.9 (split); with few solids 9.8
+  // against 10.5 at 197k, 147 against 158 at 3.96M, but 26.4 against 25.8 at 655k. FP32 fluid with FP16 thermal: 33k 4.4
+  // against 5.4, at 3.96M 126 and 141 against 136 and 146, share 0.74 at 655k 25.2 against 28.7; but 0.55 24.8 against
+  // 23.4, and 0.17 at 3.96M 123 against 96. Blocks of 128 threads for the one-pass step (64: up to 9% more at row length
+  // 128), 64 for the split step (128: 1 to 4% more).
+  void default_tune() {
+    const long long p = positions();
+    bool stage;
+    if (precision == XAC_FP32) stage = p > k1M && !split_pays();
+    else if (precision == XAC_FP32_T16) stage = p <= kSmall || share >= 0.62 || (p > k1M && share >= 0.3);
+    else stage = p <= kSmall || (share >= 0.62 && (p <= kMid || p > k1M));
+    tune_variant = stage && g.pitch <= kMaxStagedRow ? 1 : 0;
+    tune_block = tune_variant == 0 && split_pays() ? 64 : 128;
   }
   unsigned* status = nullptr;  // device word set by a step kernel whose bounded wait ran out (in red_out's tail)
   // set once the status word was seen non-zero: a staged step gave up on its copies, so the thermal populations it
@@ -450,9 +492,15 @@ struct LatticeImpl {
     return p;
   }
 
-  ~LatticeImpl() {
+  void drop_graphs() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
+    graphs.clear();
     for (auto& kv : run_graphs) cudaGraphExecDestroy(kv.second);
+    run_graphs.clear();
+  }
+
+  ~LatticeImpl() {
+    drop_graphs();
     cudaFree(run_ctl);
     if (run_ctl_host) cudaFreeHost(run_ctl_host);
     for (void* b : {P[0], P[1], Qb[0], Qb[1]}) cudaFree(b);
@@ -477,16 +525,20 @@ struct LatticeImpl {
     for (cudaEvent_t ev : events) cudaEventDestroy(ev);
   }
 
-  bool staged() const { return tune_variant == 1 && g.pitch <= kMaxStagedRow; }
-
-  void launch_staged(cudaStream_t s, bool macro, bool own) {
+  template <typename SP, typename SQ>
+  void launch_both(Form f, const StepLaunch& a) {
+    if (f == Form::kStaged) launch_staged_step<SP, SQ>(a);
+    else launch_row_step<SP, SQ>(a);
+  }
+  // one step of both lattices in one launch
+  void launch_single(Form f, cudaStream_t s, bool macro, bool own) {
     const StepLaunch a{P[cur], P[cur ^ 1], Qb[cur], Qb[cur ^ 1], link, qsrc, u_in, rho, ux, uy, uz, T, params(),
-                       macro, own, s};
+                       tune_block, macro, own, s};
     switch (precision) {
-      case XAC_FP16: launch_staged_step<__half, __half>(a); break;
-      case XAC_BF16: launch_staged_step<__nv_bfloat16, __half>(a); break;
-      case XAC_FP32_T16: launch_staged_step<float, __half>(a); break;
-      default: launch_staged_step<float, float>(a);
+      case XAC_FP16: launch_both<__half, __half>(f, a); break;
+      case XAC_BF16: launch_both<__nv_bfloat16, __half>(f, a); break;
+      case XAC_FP32_T16: launch_both<float, __half>(f, a); break;
+      default: launch_both<float, float>(f, a);
     }
     cur ^= 1;
   }
@@ -547,8 +599,9 @@ struct LatticeImpl {
 
   // n steps, the last one writing rho/u; own: the first one reads the initial thermal populations unstreamed
   void launch_steps(cudaStream_t s, int n, bool own) {
-    if (staged()) {
-      for (int k = 0; k < n; ++k) launch_staged(s, k == n - 1, own && k == 0);
+    const Form f = form(n);
+    if (f != Form::kSplit) {
+      for (int k = 0; k < n; ++k) launch_single(f, s, k == n - 1, own && k == 0);
       return;
     }
     for (int k = 1; k <= n; ++k) {
@@ -561,7 +614,7 @@ struct LatticeImpl {
   // The same with the two lattices on two branches, captured or not: thermal step k waits for fluid step k, fluid step k
   // for thermal step k - kUSets (whose velocity it overwrites). The branches join on st.
   cudaError_t branch_steps(cudaStream_t st, int n) {
-    if (staged()) {
+    if (form(n) != Form::kSplit) {
       launch_steps(st, n, false);
       return cudaSuccess;
     }
@@ -604,10 +657,11 @@ struct LatticeImpl {
   // instantiating 100 steps costs 0.5-0.9 ms, which a lattice that makes the call once would pay for nothing (the GPU is
   // no slower: launching a step takes less than running it).
   int launch_graph(cudaStream_t s, int n) {
-    XAC_CUDA(capture_streams());
     auto key = std::make_pair(n, cur);
     auto it = graphs.find(key);
-    if (it == graphs.end() && called.insert(key).second) {
+    const bool direct = it == graphs.end() && called.insert(key).second;
+    if (!direct || form(n) == Form::kSplit) XAC_CUDA(capture_streams());
+    if (direct) {
       XAC_CUDA(branch_steps(s, n));
       return XAC_OK;
     }
@@ -953,7 +1007,9 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   {
     long long words = 0;  // warps of the one-pass step that hold a non-solid cell
     for (const uint2& e : ftab) words += e.x != 0u;
-    L.default_tune(words ? (double)L.nonsolid / (32.0 * words) : 0.0);
+    L.share = (double)L.nonsolid / (double)n;
+    L.lanes = words ? (double)L.nonsolid / (32.0 * words) : 0.0;
+    L.default_tune();
   }
   const size_t p_bytes = (size_t)L.g.np * L.p_elem, q_bytes = (size_t)L.g.N * L.q_elem;
   for (int b = 0; b < 2; ++b) {
@@ -1088,6 +1144,16 @@ int xac_test_set_step_status(xac_lattice* lat, unsigned value, void* stream) {
   return XAC_OK;
 }
 
+int xac_test_step_form(xac_lattice* lat, int form) {
+  XAC_REQUIRE(lat, "xac_test_step_form: null lattice");
+  XAC_REQUIRE(form >= -1 && form <= 2 && (form != 2 || lat->impl.g.pitch <= kMaxStagedRow), "xac_test_step_form: form %d",
+              form);
+  std::lock_guard<std::mutex> g(lat->impl.mu);
+  lat->impl.drop_graphs();
+  lat->impl.forced = form;
+  return XAC_OK;
+}
+
 int xac_lattice_step(xac_lattice* lat, int n, void* stream) {
   XAC_REQUIRE(lat, "xac_lattice_step: null lattice");
   XAC_REQUIRE(n >= 0, "xac_lattice_step: negative step count %d", n);
@@ -1197,12 +1263,7 @@ int xac_lattice_tune(xac_lattice* lat, int block, int variant) {
   XAC_REQUIRE(variant == 0 || variant == 1, "xac_lattice_tune: variant must be 0 or 1 (got %d)", variant);
   LatticeImpl& L = lat->impl;
   std::lock_guard<std::mutex> g(L.mu);
-  if (L.tune_block != block || L.tune_variant != variant) {
-    for (auto& kv : L.graphs) cudaGraphExecDestroy(kv.second);
-    L.graphs.clear();
-    for (auto& kv : L.run_graphs) cudaGraphExecDestroy(kv.second);
-    L.run_graphs.clear();
-  }
+  if (L.tune_block != block || L.tune_variant != variant) L.drop_graphs();
   L.tune_block = block;
   L.tune_variant = variant;
   return XAC_OK;

@@ -610,18 +610,46 @@ __device__ __forceinline__ void pad_fill(bool valid, unsigned valid_lanes, int l
   }
 }
 
+// ---- both lattices in one pass (launch variant 0) -----------------------------------------------------------
+// One thread per row position: block-consecutive threads walk x along a row (a warp never spans
+// two rows, the row length being a multiple of 32); positions x >= nx are padding. kT > 0 makes the row length and every
+// thermal population offset compile-time constants; kT = 0 reads it from the geometry.
+template <typename SP, typename SQ, bool kMacro, bool kOwn, int kT>
+__global__ void __launch_bounds__(256) coupled_step_kernel(const SP* __restrict__ Pin, SP* __restrict__ Pout,
+                                                           const SQ* __restrict__ Qin, SQ* __restrict__ Qout,
+                                                           const uint32_t* __restrict__ link,
+                                                           const float* __restrict__ qsrc,
+                                                           const float* __restrict__ u_in_ptr,
+                                                           float* __restrict__ rho_o, float* __restrict__ ux_o,
+                                                           float* __restrict__ uy_o, float* __restrict__ uz_o,
+                                                           const float* __restrict__ T0,
+                                                           const __grid_constant__ StepParams p) {
+  const int RL = row_len<kT>(p.g);
+  const uint32_t blk = p.reverse ? gridDim.x - 1u - blockIdx.x : blockIdx.x;
+  const uint32_t pos = blk * blockDim.x + threadIdx.x;
+  const uint32_t r = pos / (uint32_t)RL, x = pos - r * (uint32_t)RL;
+  if (r >= (uint32_t)p.g.rows) return;  // whole warps
+  const int lane = threadIdx.x & 31;
+  const bool valid = x < (uint32_t)p.g.nx;
+  const uint32_t c = r * (uint32_t)p.g.nx + x;
+  const uint32_t lw = valid ? __ldg(link + c) : ((uint32_t)kSolid << kTypeShift);
+  const uint32_t e0 = pop_base(r, x, p.g, RL);
+  coupled_cell<SP, SQ, kMacro, kOwn, 0, kT>(c, r, x, e0, Pin, Pout, Qin, Qout, qsrc, u_in_ptr, rho_o, ux_o, uy_o,
+                                            uz_o, T0, p, valid, lw);
+  pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, Qout, e0, p.g);
+}
+
 // ---- the two lattices side by side (launch variant 0) ----------------------------------------------------
-// The fluid does not depend on the temperature, so the lattices run as two kernels, the fluid's a step ahead: fluid step
+// The fluid does not depend on the temperature, so the lattices can run as two kernels, the fluid's a step ahead: fluid step
 // k + 1 beside thermal step k, on two branches of the captured graph. The fluid kernel takes the non-solid cells in storage
 // order, one per thread: its warps are full, where a warp of 32 consecutive x has 43% non-solid lanes on a 57%-solid
 // gyroid. The thermal kernel takes one row position per thread and reads u by slot from one of two sets.
-// Bound: memory in FP32 (152 B per cell and 152 B per non-solid cell, and 24 B per non-solid cell for u; a plain
-// ping-pong copy of those bytes takes 21.5 us on the 148x128x32 gyroid), instruction issue in 16 bits (9.4 M + 6.2 M
-// warp instructions a step, where one pass over the row positions takes 21.8 M + conversions). Measured on that design, one
-// kernel for both lattices by row position -> this: FP32 28.5 -> 27.0 us, FP16 28.8 -> 20.5, FP32 fluid with FP16
-// thermal 27.2 -> 21.5. Tried: both lattices in one launch, fluid blocks first 33.4 (more DRAM traffic: the thermal rows of the
-// last step have left L2), with u in cell order 29.3, programmatic dependent launch -2% to +10%, thermal rows staged in
-// shared memory 27.7 / 21.7, 32 registers 28.6 / 22.6, both in one launch with alternating blocks 28.9 / 23.9.
+// Bound: instruction issue in 16 bits, memory in FP32 (152 B per cell and 152 B per non-solid cell, and 24 B per non-solid
+// cell for u). Measured on that design (655k row positions), the one-pass step -> this: FP16 26.4 -> 21.7 us, FP32 fluid with
+// FP16 thermal 26.9 -> 23.4, FP32 28.2 -> 28.5; LatticeImpl::form has the sizes and designs where it pays. Tried: both
+// lattices in one launch, fluid blocks first 33.4 in FP32 (more DRAM traffic: the thermal rows of the last step have left
+// L2), with u in cell order 29.3, programmatic dependent launch -2% to +10%, thermal rows staged in shared memory 27.7 /
+// 21.7 in FP16, 32 registers 28.6 / 22.6, both in one launch with alternating blocks 28.9 / 23.9.
 struct SplitArgs {
   const void* Pin;  // fluid step k + 1
   void* Pout;
@@ -840,7 +868,7 @@ __global__ void __launch_bounds__(kT) coupled_qstage_kernel(const SP* __restrict
   pad_fill<SQ, kT>(valid, __ballot_sync(0xffffffffu, valid), lane, Qout, e0, p.g);
 }
 
-// Arguments of one staged step launch; the launchers (step_kernels.cuh, one translation unit per storage mode) pick the
+// Arguments of one launch of the staged or the one-pass step; the launchers (step_kernels.cuh, one translation unit per storage mode) pick the
 // instantiation whose compile-time row length matches the lattice.
 struct StepLaunch {
   const void* Pin;
@@ -853,6 +881,7 @@ struct StepLaunch {
   float *rho, *ux, *uy, *uz;
   const float* T0;
   StepParams p;
+  int block;  // threads per block of the one-pass step
   bool macro, own;
   cudaStream_t stream;
 };
@@ -860,6 +889,9 @@ struct StepLaunch {
 constexpr int kMaxStagedRow = 320;
 template <typename SP, typename SQ>
 void launch_staged_step(const StepLaunch& a);
+// the one-pass step (variant 0)
+template <typename SP, typename SQ>
+void launch_row_step(const StepLaunch& a);
 // the two halves of the split step (variant 0); plain: no first step and no field output
 template <typename SP>
 void launch_split_fluid(const SplitArgs& a, int block, bool plain, cudaStream_t s);

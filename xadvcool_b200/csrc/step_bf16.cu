@@ -4,5 +4,6 @@
 
 namespace xac {
 template void launch_staged_step<__nv_bfloat16, __half>(const StepLaunch&);
+template void launch_row_step<__nv_bfloat16, __half>(const StepLaunch&);
 template void launch_split_fluid<__nv_bfloat16>(const SplitArgs&, int, bool, cudaStream_t);
 }  // namespace xac

@@ -3,6 +3,7 @@
 
 namespace xac {
 template void launch_staged_step<__half, __half>(const StepLaunch&);
+template void launch_row_step<__half, __half>(const StepLaunch&);
 template void launch_split_fluid<__half>(const SplitArgs&, int, bool, cudaStream_t);
 template void launch_split_thermal<__half>(const SplitArgs&, int, bool, cudaStream_t);
 }  // namespace xac

@@ -3,6 +3,7 @@
 
 namespace xac {
 template void launch_staged_step<float, float>(const StepLaunch&);
+template void launch_row_step<float, float>(const StepLaunch&);
 template void launch_split_fluid<float>(const SplitArgs&, int, bool, cudaStream_t);
 template void launch_split_thermal<float>(const SplitArgs&, int, bool, cudaStream_t);
 }  // namespace xac

@@ -3,4 +3,5 @@
 
 namespace xac {
 template void launch_staged_step<float, __half>(const StepLaunch&);
+template void launch_row_step<float, __half>(const StepLaunch&);
 }  // namespace xac

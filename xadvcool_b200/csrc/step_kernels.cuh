@@ -39,6 +39,35 @@ void launch_staged_step(const StepLaunch& a) {
   else launch_staged_rows<SP, SQ, false, false>(a);
 }
 
+template <typename SP, typename SQ, bool kMacro, bool kOwn>
+void launch_rows(const StepLaunch& a) {
+  const unsigned grid = (unsigned)(((long long)a.p.g.rows * a.p.g.pitch + a.block - 1) / a.block);
+#define XAC_STEP(KT)                                                                                             \
+  coupled_step_kernel<SP, SQ, kMacro, kOwn, KT><<<grid, a.block, 0, a.stream>>>(                                  \
+      (const SP*)a.Pin, (SP*)a.Pout, (const SQ*)a.Qin, (SQ*)a.Qout, a.link, a.qsrc, a.u_in, a.rho, a.ux, a.uy,    \
+      a.uz, a.T0, a.p)
+  switch (a.p.g.pitch) {
+    case 32: XAC_STEP(32); return;
+    case 64: XAC_STEP(64); return;
+    case 96: XAC_STEP(96); return;
+    case 128: XAC_STEP(128); return;
+    case 160: XAC_STEP(160); return;
+    case 192: XAC_STEP(192); return;
+    case 224: XAC_STEP(224); return;
+    case 256: XAC_STEP(256); return;
+    default: XAC_STEP(0);
+  }
+#undef XAC_STEP
+}
+
+template <typename SP, typename SQ>
+void launch_row_step(const StepLaunch& a) {
+  if (a.macro && a.own) launch_rows<SP, SQ, true, true>(a);
+  else if (a.macro) launch_rows<SP, SQ, true, false>(a);
+  else if (a.own) launch_rows<SP, SQ, false, true>(a);
+  else launch_rows<SP, SQ, false, false>(a);
+}
+
 template <typename SP>
 void launch_split_fluid(const SplitArgs& a, int block, bool plain, cudaStream_t s) {
   const unsigned grid = a.fblocks + a.eblocks;

@@ -102,8 +102,9 @@ class Lattice:
         return int(v.value)
 
     def tune(self, block: int, variant: int):
-        """Launch shape of the step: threads per block (64, 128, 256) and variant (0: fluid and thermal lattice in
-        kernels of their own; 1: one block per row with the thermal input staged in shared memory). Results are unaffected."""
+        """Launch shape of the step: threads per block (64, 128, 256) and variant (0: one thread per row
+        position, or fluid and thermal lattice in kernels of their own; 1: one block per row with the thermal input staged
+        in shared memory). Results are unaffected."""
         _capi.call("xac_lattice_tune", self._h, int(block), int(variant))
 
     def pattern_copy_us(self, launches: int = 200) -> float:
