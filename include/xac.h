@@ -167,6 +167,9 @@ int xac_test_dirichlet_plane(float *g, float T_val, int x_plane, int nx, int ny,
  * polls (1..2^20). status_out: bit 0 the mbarrier wait gave up, bit 1 the grid barrier gave up, bit 2 the grid
  * barrier recorded XAC_ETIMEOUT; 7 when every wait reported. The context stays usable. */
 int xac_test_bounded_waits(unsigned limit, unsigned *status_out, void *stream);
+/* Test hook: a block at the batch kernel's grid barrier that nobody completes, after another block has recorded that its
+ * wait gave up; milliseconds until it leaves. */
+int xac_test_barrier_after_error(unsigned limit, float *ms, void *stream);
 /* Test-only: the convolution kernels' mbarrier wait on a barrier nothing completes, limited to `limit` polls
  * (1..2^20); it must set bit 0 of the flags xac_conv3d_status returns. */
 int xac_test_conv_wait_timeout(unsigned limit, void *stream);

@@ -105,6 +105,7 @@ SIGNATURES = {
     "xac_thermal_macroscopic": [_vp, _vp, _i, _i, _i, _vp],
     "xac_test_dirichlet_plane": [_vp, _f, _i, _i, _i, _i, _vp],
     "xac_test_bounded_waits": [C.c_uint, _vp, _vp],
+    "xac_test_barrier_after_error": [C.c_uint, C.POINTER(_f), _vp],
     "xac_test_set_step_status": [_vp, C.c_uint, _vp],
     "xac_test_step_form": [_vp, _i],
     "xac_test_conv_wait_timeout": [C.c_uint, _vp],

@@ -87,8 +87,10 @@ __device__ __forceinline__ bool grid_sync(BatchCtl* ctl, unsigned long long spin
     if (!released) {
       unsigned long long spins = 0;
       while (*gen == g) {
-        if (++spins > spin_limit) {
-          atomicExch(&ctl->err, XAC_ETIMEOUT);
+        // once one block has given up the others need not wait as long: the error is looked at every 1024 polls
+        const bool late = ++spins > spin_limit;
+        if (late) atomicExch(&ctl->err, XAC_ETIMEOUT);
+        if (late || ((spins & 1023u) == 0 && *(volatile int*)&ctl->err)) {
           ok = false;
           break;
         }
@@ -97,7 +99,7 @@ __device__ __forceinline__ bool grid_sync(BatchCtl* ctl, unsigned long long spin
     }
     __threadfence();
   }
-  // a block whose wait ran out leaves; the others' next wait then runs out too
+  // a block whose wait ran out leaves, and the others out of their next wait
   return __syncthreads_and(ok) != 0;
 }
 

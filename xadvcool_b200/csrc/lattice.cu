@@ -1450,6 +1450,33 @@ extern "C" int xac_test_bounded_waits(unsigned limit, unsigned* status_out, void
   return XAC_OK;
 }
 
+// The same meeting with the error already recorded: the wait ends long before its limit. Device time of the launch.
+extern "C" int xac_test_barrier_after_error(unsigned limit, float* ms, void* stream) {
+  XAC_REQUIRE(ms, "xac_test_barrier_after_error: null pointer");
+  XAC_REQUIRE(limit > 0 && limit <= (1u << 20), "xac_test_barrier_after_error: limit %u out of (0, 2^20]", limit);
+  cudaStream_t s = as_stream(stream);
+  BatchCtl* ctl = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  XAC_CUDA(cudaMalloc(&ctl, sizeof(BatchCtl) + sizeof(unsigned)));
+  const int err = XAC_ETIMEOUT;
+  cudaError_t e = cudaMemsetAsync(ctl, 0, sizeof(BatchCtl) + sizeof(unsigned), s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&ctl->err, &err, sizeof(err), cudaMemcpyHostToDevice, s);
+  for (cudaEvent_t& v : ev)
+    if (e == cudaSuccess) e = cudaEventCreate(&v);
+  if (e == cudaSuccess) e = cudaEventRecord(ev[0], s);
+  if (e == cudaSuccess) {
+    test_grid_barrier_timeout_kernel<<<2, 32, 0, s>>>(ctl, (unsigned long long)limit, (unsigned*)(ctl + 1));
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaEventRecord(ev[1], s);
+  if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
+  if (e == cudaSuccess) e = cudaEventElapsedTime(ms, ev[0], ev[1]);
+  for (cudaEvent_t v : ev)
+    if (v) cudaEventDestroy(v);
+  cudaFree(ctl);
+  return e == cudaSuccess ? XAC_OK : cuda_status(e, "xac_test_barrier_after_error");
+}
+
 // simulation.py:102-162
 int xac_lattice_run(xac_lattice* lat, const xac_run_opts* o, xac_run_result* res, void* stream) {
   XAC_REQUIRE(lat && o && res, "xac_lattice_run: null pointer");
