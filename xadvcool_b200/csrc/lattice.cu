@@ -432,11 +432,13 @@ struct LatticeImpl {
   uint32_t* link = nullptr;
   uint2* ftab = nullptr;  // non-solid cell table of the fluid populations
   uint32_t nonsolid = 0;  // non-solid cells (the fluid populations' slots in use)
-  uint2* cells = nullptr;    // the split step's non-solid cells, by slot
+  std::vector<uint32_t> ends_host;  // slots of the inlet and outlet cells
+  // What only the split step needs, in one allocation that starts at u_step: lattices on the other forms and the designs of
+  // a batch do without its 32 bytes per non-solid cell.
+  uint2* cells = nullptr;    // the non-solid cells, by slot
   uint32_t* ends = nullptr;  // slots of the inlet and outlet cells
-  uint32_t nends = 0;
   static constexpr int kUSets = 2;  // three sets measured the same
-  float* u_step = nullptr;  // [kUSets][3][ncell]: u by slot, from the fluid's step to the thermal lattice's
+  float* u_step = nullptr;  // [kUSets][3][ns]: u by slot, from the fluid's step to the thermal lattice's
   float* qsrc = nullptr;
   float* u_in = nullptr;
   float *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr, *T = nullptr;
@@ -507,8 +509,6 @@ struct LatticeImpl {
     cudaFree(type);
     cudaFree(link);
     cudaFree(ftab);
-    cudaFree(cells);
-    cudaFree(ends);
     cudaFree(u_step);
     cudaFree(qsrc);
     cudaFree(u_in);
@@ -543,13 +543,46 @@ struct LatticeImpl {
     cur ^= 1;
   }
 
+  // The split step's memory, before its first run. A caller's capture of s goes on undisturbed: the memory is made outside it.
+  int need_split(cudaStream_t s) {
+    if (u_step) return XAC_OK;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    XAC_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs == cudaStreamCaptureStatusNone) return make_split(s);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    XAC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = capture_streams();
+    const int r = e == cudaSuccess ? make_split(fluid_branch) : cuda_status(e, "streams of the split step");
+    XAC_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    return r;
+  }
+  int make_split(cudaStream_t s) {
+    const size_t ub = (size_t)kUSets * 3 * g.ns * sizeof(float), cb = (size_t)g.ns * sizeof(uint2);
+    const size_t eb = ends_host.size() * sizeof(uint32_t);
+    char* m = nullptr;
+    int r = dmalloc(&m, ub + cb + eb, "alloc split step");
+    if (r != XAC_OK) return r;
+    cells = reinterpret_cast<uint2*>(m + ub);
+    ends = reinterpret_cast<uint32_t*>(m + ub + cb);
+    cudaError_t e = eb ? cudaMemcpyAsync(ends, ends_host.data(), eb, cudaMemcpyHostToDevice, s) : cudaSuccess;
+    build_cells_kernel<<<grid_for(g.ncell, kBlock), kBlock, 0, s>>>(link, ftab, cells, g);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      cudaFree(m);
+      return cuda_status(e, "split step's lists");
+    }
+    u_step = reinterpret_cast<float*>(m);
+    return XAC_OK;
+  }
+
   // One launch of the split step in a run of n: the fluid lattice's step f (1..n, 0: none) and the thermal lattice's step
   // t (0: none). c0 is the buffer parity before the run. The last step also writes rho and u to the field arrays.
   void launch_split(cudaStream_t s, int n, int c0, int f, int t, bool own) {
     SplitArgs a{};
     const int cf = (c0 + f + 1) & 1, ct = (c0 + t + 1) & 1;  // parity of the buffers step f / t reads
     float* const field[3] = {ux, uy, uz};
-    auto uset = [&](int back, int k) { return u_step + ((size_t)(back % kUSets) * 3 + k) * g.ncell; };
+    auto uset = [&](int back, int k) { return u_step + ((size_t)(back % kUSets) * 3 + k) * g.ns; };
     a.p = params();
     a.tab = tables();
     a.link = link;
@@ -559,13 +592,13 @@ struct LatticeImpl {
     a.ends = ends;
     a.T0 = T;
     a.nfluid = nonsolid;
-    a.nends = nends;
+    a.nends = (uint32_t)ends_host.size();
     const unsigned B = (unsigned)tune_block;
     if (f > 0) {
       a.Pin = P[cf];
       a.Pout = P[cf ^ 1];
       a.fblocks = (nonsolid + B - 1) / B;
-      a.eblocks = (nends + B - 1) / B;
+      a.eblocks = (a.nends + B - 1) / B;
       a.frev = (uint32_t)cf;
       if (f == n) {
         a.field[0] = rho;
@@ -694,6 +727,10 @@ struct LatticeImpl {
   int steps(int n, cudaStream_t s) {
     if (n <= 0) return XAC_OK;
     if (staged()) XAC_CUDA(note_staged(s));
+    if (form(1) == Form::kSplit || form(n) == Form::kSplit) {
+      const int r = need_split(s);
+      if (r != XAC_OK) return r;
+    }
     if (own_pending) {
       launch_steps(s, 1, true);
       own_pending = false;
@@ -723,7 +760,11 @@ struct LatticeImpl {
   // The device-resident run loop for the current buffer parity: a graph whose while node repeats
   // { every plain steps, T, stats, run_decision_kernel } until the decision kernel clears the condition.
   // every must be even (the parity is the same at each iteration).
-  int run_graph(int every, cudaGraphExec_t* out) {
+  int run_graph(int every, cudaGraphExec_t* out, cudaStream_t s) {
+    if (form(every) == Form::kSplit) {
+      const int r = need_split(s);
+      if (r != XAC_OK) return r;
+    }
     auto key = std::make_pair(every, cur);
     auto it = run_graphs.find(key);
     if (it != run_graphs.end()) {
@@ -1001,9 +1042,7 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
         type[((size_t)z * ny + y) * nx + x] = (uint8_t)m;
       }
   std::vector<float> q = host_qsrc(d);
-  std::vector<uint32_t> ends;
-  const std::vector<uint2> ftab = fluid_table(type.data(), L.g, &L.nonsolid, &ends);
-  L.nends = (uint32_t)ends.size();
+  const std::vector<uint2> ftab = fluid_table(type.data(), L.g, &L.nonsolid, &L.ends_host);
   {
     long long words = 0;  // warps of the one-pass step that hold a non-solid cell
     for (const uint2& e : ftab) words += e.x != 0u;
@@ -1020,9 +1059,6 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   if ((r = dmalloc(&L.type, n, "alloc type")) != XAC_OK) return r;
   if ((r = dmalloc(&L.link, n, "alloc link")) != XAC_OK) return r;
   if ((r = dmalloc(&L.ftab, ftab.size(), "alloc fluid table")) != XAC_OK) return r;
-  if ((r = dmalloc(&L.cells, n, "alloc cell list")) != XAC_OK) return r;
-  if ((r = dmalloc(&L.ends, ends.size(), "alloc inlet and outlet list")) != XAC_OK) return r;
-  if ((r = dmalloc(&L.u_step, 3 * LatticeImpl::kUSets * (size_t)n, "alloc velocity")) != XAC_OK) return r;
   if ((r = dmalloc(&L.qsrc, n, "alloc qsrc")) != XAC_OK) return r;
   if ((r = dmalloc(&L.u_in, 1, "alloc u_in")) != XAC_OK) return r;
   for (float** f : {&L.rho, &L.ux, &L.uy, &L.uz, &L.T})
@@ -1044,13 +1080,10 @@ int create_impl(const xac_desc* d, LatticeImpl& L, cudaStream_t s) {
   XAC_CUDA(cudaMemcpyAsync(L.type, type.data(), n, cudaMemcpyHostToDevice, s));
   XAC_CUDA(cudaMemcpyAsync(L.ftab, ftab.data(), ftab.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
   XAC_CUDA(cudaMemcpyAsync(L.qsrc, q.data(), n * sizeof(float), cudaMemcpyHostToDevice, s));
-  if (!ends.empty())
-    XAC_CUDA(cudaMemcpyAsync(L.ends, ends.data(), ends.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
   set_scalar_kernel<<<1, 1, 0, s>>>(L.u_in, L.u_in_host);
   relaxation_factors_kernel<<<1, 1, 0, s>>>((float)L.tau_fluid, L.tau_th_f, L.tau_th_s, (float*)L.red_out);
   XAC_CUDA(cudaMemcpyAsync(L.relax, L.red_out, sizeof(L.relax), cudaMemcpyDeviceToHost, s));
   build_link_kernel<<<grid_for(n, kBlock), kBlock, 0, s>>>(L.type, L.qsrc, L.link, L.g);
-  build_cells_kernel<<<grid_for(n, kBlock), kBlock, 0, s>>>(L.link, L.ftab, L.cells, L.g);
   XAC_CUDA(cudaGetLastError());
   // host vectors go out of scope: make the copies complete first
   XAC_CUDA(cudaStreamSynchronize(s));
@@ -1092,6 +1125,27 @@ int init_impl(LatticeImpl& L, const float* rho, const float* u, const float* T, 
   return XAC_OK;
 }
 
+// alone: the lattice is stepped by itself, not by a batch
+int create_lattice(const xac_desc* desc, xac_lattice** out, cudaStream_t s, bool alone) {
+  XAC_REQUIRE(out, "xac_lattice_create: null output handle");
+  *out = nullptr;
+  xac_lattice* lat = new (std::nothrow) xac_lattice();
+  if (!lat) {
+    set_error("xac_lattice_create: host allocation failed");
+    return XAC_ENOMEM;
+  }
+  int r = create_impl(desc, lat->impl, s);
+  if (r == XAC_OK) r = init_impl(lat->impl, nullptr, nullptr, nullptr, s);
+  if (r == XAC_OK && alone && lat->impl.form(LatticeImpl::kGraphSteps) == LatticeImpl::Form::kSplit)
+    r = lat->impl.need_split(s);
+  if (r != XAC_OK) {
+    delete lat;
+    return r;
+  }
+  *out = lat;
+  return XAC_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1100,22 +1154,7 @@ const char* xac_last_error(void) { return xac::g_err; }
 int xac_version(void) { return 10000; }
 
 int xac_lattice_create(const xac_desc* desc, xac_lattice** out, void* stream) {
-  XAC_REQUIRE(out, "xac_lattice_create: null output handle");
-  *out = nullptr;
-  xac_lattice* lat = new (std::nothrow) xac_lattice();
-  if (!lat) {
-    set_error("xac_lattice_create: host allocation failed");
-    return XAC_ENOMEM;
-  }
-  cudaStream_t s = as_stream(stream);
-  int r = create_impl(desc, lat->impl, s);
-  if (r == XAC_OK) r = init_impl(lat->impl, nullptr, nullptr, nullptr, s);
-  if (r != XAC_OK) {
-    delete lat;
-    return r;
-  }
-  *out = lat;
-  return XAC_OK;
+  return create_lattice(desc, out, as_stream(stream), true);
 }
 
 int xac_lattice_destroy(xac_lattice* lat) {
@@ -1535,7 +1574,7 @@ int xac_lattice_run(xac_lattice* lat, const xac_run_opts* o, xac_run_result* res
       cudaStream_t s = as_stream(stream);
       std::lock_guard<std::mutex> g(L.mu);
       cudaGraphExec_t ex = nullptr;
-      r = L.run_graph(o->stats_every, &ex);
+      r = L.run_graph(o->stats_every, &ex, s);
       if (r != XAC_OK) return r;
       RunCtl& c = *L.run_ctl_host;
       std::memset(&c, 0, sizeof(c));
@@ -1870,7 +1909,7 @@ int xac_batch_create(const xac_desc* descs, int n, xac_batch** out, void* stream
   b->precision = descs[0].precision;
   for (int i = 0; i < n; ++i) {
     xac_lattice* l = nullptr;
-    int r = xac_lattice_create(&descs[i], &l, stream);
+    int r = create_lattice(&descs[i], &l, as_stream(stream), false);
     if (r != XAC_OK) {
       delete b;
       return r;
@@ -2034,7 +2073,7 @@ int xac_batch_admit(xac_batch* b, const xac_desc* desc, int* slot, void* stream)
   while (k < (int)b->lats.size() && b->state[k] != xac_batch::kFree) ++k;
   XAC_REQUIRE(k < kMaxBatch, "xac_batch_admit: all %d slots hold designs (release finished ones first)", kMaxBatch);
   xac_lattice* l = nullptr;
-  int r = xac_lattice_create(desc, &l, stream);
+  int r = create_lattice(desc, &l, as_stream(stream), false);
   if (r != XAC_OK) return r;
   if (k == (int)b->lats.size()) {
     b->lats.push_back(nullptr);
@@ -2159,7 +2198,7 @@ int xac_batch_advance(xac_batch* b, const xac_run_opts* o, long long steps, int*
   return XAC_OK;
 }
 
-// Device bytes a lattice of this descriptor allocates (populations, link words, fields, reduction rows).
+// Device bytes a lattice of this descriptor allocates in a batch (populations, link words, fields, reduction rows).
 int xac_lattice_footprint(const xac_desc* d, unsigned long long* bytes) {
   XAC_REQUIRE(d && bytes, "xac_lattice_footprint: null pointer");
   XAC_REQUIRE(d->nx >= 1 && d->ny >= 1 && d->nz >= 1, "xac_lattice_footprint: bad lattice size");
@@ -2167,21 +2206,17 @@ int xac_lattice_footprint(const xac_desc* d, unsigned long long* bytes) {
   const long long pitch = (d->nx + 31) / 32 * 32;
   const long long N = ((long long)d->ny * d->nz + 2LL * (d->ny + 2)) * kQ * pitch;
   // fluid populations of the non-solid cells (all cells when no mask is given)
-  long long nonsolid = n, ends = 0;
+  long long nonsolid = n;
   if (d->mask) {
     nonsolid = 0;
-    for (long long c = 0; c < n; ++c) {
-      nonsolid += d->mask[c] != kSolid;
-      ends += d->mask[c] == kInlet || d->mask[c] == kOutlet;
-    }
+    for (long long c = 0; c < n; ++c) nonsolid += d->mask[c] != kSolid;
   }
   const long long NP = kQ * ((nonsolid + 31) / 32 * 32 + (nonsolid == 0 ? 32 : 0));
   const long long ftab = ((long long)d->ny * d->nz + 2LL * (d->ny + 1)) * (pitch / 32) * 8;
   const long long p_elem = (d->precision == XAC_FP32 || d->precision == XAC_FP32_T16) ? 4 : 2;
   const long long q_elem = d->precision == XAC_FP32 ? 4 : 2;
   const long long metric_rows = (long long)reduction_blocks(n) * kNMetrics, stat_rows = stats_tiles(n) * kNStats;
-  *bytes = (unsigned long long)(2 * NP * p_elem + 2 * N * q_elem + ftab + 4 * ends +
-                                n * (1 + 4 + 4 + 8 + 5 * 4 + 6 * 4) +
+  *bytes = (unsigned long long)(2 * NP * p_elem + 2 * N * q_elem + ftab + n * (1 + 4 + 4 + 5 * 4) +
                                 8 * (metric_rows > stat_rows ? metric_rows : stat_rows) + 64 * 8 + 64);
   return XAC_OK;
 }
