@@ -334,6 +334,7 @@ struct LatticeImpl {
   float relax[5] = {1.0f, 1.0f, 1.0f, 0.5f, 0.5f};  // omega_f, omega_tf, omega_ts, srcf_f, srcf_s (device-computed)
   float u_in_host = 0.0f;
   int tune_block = 128;  // threads per block of the one-pass step and of the split step's kernels
+  bool tuned = false;    // by a caller; otherwise short runs beside split ones take 128 too
   int tune_variant = 0;  // 0: one-pass or split step, by form(); 1: thermal rows staged in shared memory
   double share = 1.0, lanes = 1.0;  // non-solid cells, of all cells and of the lanes of warps that hold one
   long long positions() const { return (long long)g.rows * g.pitch; }
@@ -379,6 +380,7 @@ struct LatticeImpl {
   // against 5.4, at 3.96M 126 and 141 against 136 and 146, share 0.74 at 655k 25.2 against 28.7; but 0.55 24.8 against
   // 23.4, and 0.17 at 3.96M 123 against 96. Blocks of 128 threads for the one-pass step (64: up to 9% more at row length
   // 128), 64 for the split step (128: 1 to 4% more).
+  int row_block() const { return tuned ? tune_block : 128; }
   void default_tune() {
     const long long p = positions();
     bool stage;
@@ -533,7 +535,7 @@ struct LatticeImpl {
   // one step of both lattices in one launch
   void launch_single(Form f, cudaStream_t s, bool macro, bool own) {
     const StepLaunch a{P[cur], P[cur ^ 1], Qb[cur], Qb[cur ^ 1], link, qsrc, u_in, rho, ux, uy, uz, T, params(),
-                       tune_block, macro, own, s};
+                       row_block(), macro, own, s};
     switch (precision) {
       case XAC_FP16: launch_both<__half, __half>(f, a); break;
       case XAC_BF16: launch_both<__nv_bfloat16, __half>(f, a); break;
@@ -687,8 +689,10 @@ struct LatticeImpl {
   }
 
   // n >= 8 plain steps. The first call of a length launches them one by one, later ones from a graph: capturing and
-  // instantiating 100 steps costs 0.5-0.9 ms, which a lattice that makes the call once would pay for nothing (the GPU is
-  // no slower: launching a step takes less than running it).
+  // instantiating 100 steps costs 0.3 ms in one launch a step and 0.9 ms in two, which a program that makes the call once
+  // (xac_lattice_run's first interval, for one) would pay for nothing. One that repeats it pays more in all: 100 steps at 33k
+  // row positions in FP32, where the host takes 6 us a launch and the GPU 4.3 a step, take 0.63, 0.96, then 0.42 ms a call,
+  // with a graph at once 0.87, 0.45, 0.43; the split step at 655k in FP16 2.64, 3.29, then 2.17.
   int launch_graph(cudaStream_t s, int n) {
     auto key = std::make_pair(n, cur);
     auto it = graphs.find(key);
@@ -1302,7 +1306,8 @@ int xac_lattice_tune(xac_lattice* lat, int block, int variant) {
   XAC_REQUIRE(variant == 0 || variant == 1, "xac_lattice_tune: variant must be 0 or 1 (got %d)", variant);
   LatticeImpl& L = lat->impl;
   std::lock_guard<std::mutex> g(L.mu);
-  if (L.tune_block != block || L.tune_variant != variant) L.drop_graphs();
+  if (L.tune_block != block || L.tune_variant != variant || !L.tuned) L.drop_graphs();
+  L.tuned = true;
   L.tune_block = block;
   L.tune_variant = variant;
   return XAC_OK;
@@ -1919,8 +1924,10 @@ int xac_batch_create(const xac_desc* descs, int n, xac_batch** out, void* stream
   size_t rows = 0;
   for (auto* l : b->lats) rows += (size_t)stats_tiles(l->impl.g.ncell);
   b->rows_cap = rows;
-  // fewer, larger blocks meet sooner where the barrier counts (255k cells: 26.6 us a step at 256 threads, 27.7 at 128); where
-  // the sweep does, 128 is the better tile (964k cells: 68.5 against 66.1)
+  // Fewer, larger blocks meet sooner where the barrier counts: 64 designs, 498k row positions 36.6 us a step at 256 threads,
+  // 40.5 at 128 (FP16 40.7, 44.8), 16 designs, 345k 26.8, 26.9 (29.6, 30.5); two designs of 380k lose, 32.7 against 31.4.
+  // Where the sweep counts, 128 is the better tile: 650k 46.7 against 46.3, 689k 47.0, 45.5, 969k 63.2, 62.2. The cut is four
+  // tiles for each of the 592 blocks of 256 threads that 148 SMs hold. An open batch stays at 128: its designs come and go.
   long long positions = 0;
   for (auto* l : b->lats) positions += (long long)l->impl.g.rows * l->impl.g.pitch;
   if (positions <= 4LL * 148 * 4 * 256) b->block = 256;
