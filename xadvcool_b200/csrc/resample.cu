@@ -4,7 +4,8 @@
 //
 // What bounds them: memory, one read of each input and one write of each output. A thread takes an octet of channels (16
 // bytes) of one coarse voxel, or of one fine voxel of the joined volume; eight values are added in FP32 and rounded to
-// BF16 once, in any order the same on activations of this network. The tensor operations this replaces wrote FP32 copies of
+// BF16 once. Where their exponents lie within 13 bits of one another the sum is exact in any order; others round by the
+// order, and gave the tensor operations' bits on the cases measured. The tensor operations this replaces wrote FP32 copies of
 // the fine volume and the upsampled volume on its own: a training step's gradients at batch 4 10.8 -> 9.7 ms, a prediction
 // 2.97 -> 2.69.
 #include <cuda_bf16.h>
