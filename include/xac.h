@@ -173,6 +173,10 @@ int xac_test_barrier_after_error(unsigned limit, float *ms, void *stream);
 /* Test-only: the convolution kernels' mbarrier wait on a barrier nothing completes, limited to `limit` polls
  * (1..2^20); it must set bit 0 of the flags xac_conv3d_status returns. */
 int xac_test_conv_wait_timeout(unsigned limit, void *stream);
+/* Test hook: the tiles chosen for a shape on `sms` SMs (host only). fwd[8]: units, CTAs, planes kept, planes held, weights
+ * resident, weight stages, accumulator buffers, accumulator blocks; wg[7]: units, CTAs, planes kept, planes held, units of an
+ * accumulation, accumulator buffers, d_out copied by rows. */
+int xac_test_conv_plan(int N, int D, int H, int W, int Ci, int Co, int ksize, int sms, long long *fwd, long long *wg);
 /* validate_analytical.py:255-273 periodic_streaming_kernel and :607-621 periodic_thermal_streaming_kernel */
 int xac_test_periodic_stream(const float *f_post, float *f_streamed, int nx, int ny, int nz, void *stream);
 /* validate_analytical.py:377-395 forced_bgk_collision_kernel(f_old, f_eq, f_new, mask, tau, force_x) */

@@ -109,6 +109,7 @@ SIGNATURES = {
     "xac_test_set_step_status": [_vp, C.c_uint, _vp],
     "xac_test_step_form": [_vp, _i],
     "xac_test_conv_wait_timeout": [C.c_uint, _vp],
+    "xac_test_conv_plan": [_i] * 8 + [C.POINTER(C.c_longlong)] * 2,
     "xac_test_periodic_stream": [_vp, _vp, _i, _i, _i, _vp],
     "xac_test_forced_bgk": [_vp, _vp, _vp, _vp, _f, _f, _i, _i, _i, _vp],
     "xac_test_periodic_stream_solids": [_vp, _vp, _vp, _i, _i, _i, _vp],

@@ -1097,7 +1097,8 @@ bool search_fwd_plan(const ConvShape& s, int sms, FwdPlan* best) {
   return std::isfinite(best_cost);
 }
 
-// Plans kept by shape (the search takes some tens of microseconds); the map is emptied when it holds 256.
+// Plans kept by shape (the search takes 20 to 300 us on a host core, most for wide volumes of few channels); the map is
+// emptied when it holds 256.
 int fwd_plan(const ConvShape& s, FwdPlan* out) {
   static std::mutex mu;
   static std::map<std::array<int, 8>, FwdPlan> plans;
@@ -1336,6 +1337,21 @@ static __global__ void test_conv_wait_timeout_kernel(uint32_t limit) {
     mbar_wait(b, 0, limit);
     asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(b) : "memory");
   }
+}
+
+int xac_test_conv_plan(int N, int D, int H, int W, int Ci, int Co, int ksize, int sms, long long* fwd, long long* wg) {
+  XAC_REQUIRE(fwd && wg && sms > 0, "xac_test_conv_plan: bad arguments");
+  const ConvShape s{N, D, H, W, Ci, Co, ksize};
+  int r = check_shape(s);
+  if (r != XAC_OK) return r;
+  FwdPlan f;
+  WgPlan w;
+  XAC_REQUIRE(search_fwd_plan(s, sms, &f) && search_wg_plan(s, &w), "xac_test_conv_plan: no tile");
+  const long long a[] = {f.units, f.ctas, f.march, f.NS, f.resident, f.bs, f.nbuf, f.mt};
+  const long long b[] = {w.units, w.ctas, w.march, w.NX, w.upc, w.nbuf, w.rows_mode};
+  for (int k = 0; k < 8; ++k) fwd[k] = a[k];
+  for (int k = 0; k < 7; ++k) wg[k] = b[k];
+  return XAC_OK;
 }
 
 int xac_test_conv_wait_timeout(unsigned limit, void* stream) {
