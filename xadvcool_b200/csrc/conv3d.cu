@@ -523,10 +523,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) conv_fwd_kernel(const __grid_c
       mbar_arrive(bar.cempty(buf));
     }
   }
-  // Every MMA issued has finished before the tensor memory goes back. Only the warps that issue them wait on done, so its
-  // limit counts from the end of their own work; the others stand at the barrier, where a long launch is no failure.
+  // Every MMA issued has finished before the tensor memory goes back. The warps that work to the end wait on done, so its
+  // limit counts from the end of their own work; those that are idle or end early stand at the barrier, where a long launch
+  // is no failure. (With the MMA warps alone on done: 16 -> 16 channels at 32x128x152 34.93 us, against 34.83.)
   __syncwarp();
-  if (warp >= kEpiWarps && warp < kEpiWarps + nmw) mbar_wait(bar.done(), 0);
+  if (warp < kEpiWarps + nmw) mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) conv_wgrad_kernel(const __grid_
     }
   }
   __syncwarp();
-  if (warp >= kWgEpiWarps && warp < kWgEpiWarps + nmw) mbar_wait(bar.done(), 0);
+  if (warp < kWgEpiWarps + nmw) mbar_wait(bar.done(), 0);
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
