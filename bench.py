@@ -256,7 +256,8 @@ def run_reference_arm(args):
 
 
 # ------------------------------------------------------------------------------------------------ GPU
-STEP_KERNELS = {0: "split_fluid_kernel<float> + split_thermal_kernel<float>", 1: "coupled_qstage_kernel<float>"}
+# the step's kernel by launch variant: FP32 gyroids of this size take the one-pass form of variant 0
+STEP_KERNELS = {0: "coupled_step_kernel<float>", 1: "coupled_qstage_kernel<float>"}
 # The first of the benchmark gyroid seeds 0-23 whose cold solve reaches residual 1e-6 within 30000 steps (19,800
 # steps; seed 0 stops at the step limit, 11 of the 24 trip the divergence guard at the first check).
 CONVERGED_SEED = 15
@@ -487,7 +488,7 @@ def run_gpu_arm(args):
     achieved = alg_bytes / (step_ms * 1e-3) / 1e9
     peak, peak_kind = hbm_peak()
     tpc, tpc_why = ncu_traffic_per_cell(shape["block"], shape["variant"])
-    # the floor of the step's memory access pattern on this design: the same loads and stores, no arithmetic
+    # what the one-pass step's memory access pattern takes on this design: the same loads and stores, no arithmetic
     pattern_us = lat.pattern_copy_us(launches=5 * STEPS_PER_BENCH_STEP)
     # both buffers of the fluid and thermal populations (the state without its header and five fields)
     pop_mb = 2 * (lat.state_bytes() - 64 - 5 * 4 * cells) / 1e6
@@ -548,16 +549,17 @@ def run_gpu_arm(args):
                              "alg_bytes_per_launch": alg_bytes, "mean_launch_us": round(step_ms * 1e3, 3),
                              "pattern_floor": {"us_per_launch": round(pattern_us, 3),
                                                "step_frac": round(pattern_us / (step_ms * 1e3), 4),
-                                               "what": "the step's loads and stores (same addresses: fluid "
-                                                       "slots of the non-solid cells, thermal rows and padding "
-                                                       "fills) with no arithmetic, timed on the same lattice: "
-                                                       "step_frac = floor / step time"}},
+                                               "what": "the one-pass step's loads and stores (same addresses: "
+                                                       "fluid slots of the non-solid cells, thermal rows and "
+                                                       "padding fills) with no arithmetic, timed on the same "
+                                                       "lattice; another form's access pattern may be faster: "
+                                                       "step_frac = probe / step time"}},
                 "e2e": {"value": round(e2e_value, 2), "unit": UNIT, "h2d_bytes_per_step": h2d,
                         "d2h_bytes_per_step": d2h, "s_per_solve": round(e2e_max, 4),
                         "solves_s": [round(x, 4) for x in solve_s],
                         "solver_steps": res["steps"], "converged": res["converged"],
                         "converged_design": conv_e2e},
-                "gpu_launches": args.steps * (STEPS_PER_BENCH_STEP * (2 if shape["variant"] == 0 else 1) + 3),
+                "gpu_launches": args.steps * (STEPS_PER_BENCH_STEP + 3),
                 "launch_shape": {"block": shape["block"], "variant": shape["variant"], "autotuned": shape["table"]},
                 "forms": forms,
                 "clocks": clk.summary(),

@@ -248,8 +248,8 @@ int xac_lattice_steps_done(const xac_lattice *lat, long long *steps);
  * depend on the shape (every cell runs the same arithmetic); xadvcool_b200.autotune picks it. */
 int xac_lattice_tune(xac_lattice *lat, int block, int variant);
 int xac_lattice_get_tune(const xac_lattice *lat, int *block, int *variant);
-/* Diagnostic, no reference counterpart: the floor that the fused step's memory access pattern sets for this
- * lattice. Times `launches` launches of a kernel with the step's threads (the lattice's block size, one thread per
+/* Diagnostic, no reference counterpart: what the one-pass step's memory access pattern takes on this lattice.
+ * Times `launches` launches of a kernel with that step's threads (the lattice's block size, one thread per
  * row position, the alternating sweep), link-word and slot-table reads, population addresses (fluid pulls of the
  * non-solid cells with the bounce-back reads, thermal pulls, thermal padding fills) and no arithmetic: each value
  * read is stored unchanged. CUDA events on `stream`, after 4 untimed launches. The copies are not a physical state,
@@ -441,7 +441,8 @@ int xac_batch_launch_counts(const xac_batch *batch, long long *graph_launches, l
  * gpu_seconds must hold xac_batch_size() entries. A finished design keeps its lattice (xac_batch_lattice: fields,
  * stats, scalars) until xac_batch_release frees its slot and device memory. xac_lattice_footprint gives the
  * device bytes a design will take, for admission under a memory budget; it reads design->mask when given, since
- * fluid populations are stored for the non-solid cells only (without a mask every cell counts). */
+ * fluid populations are stored for the non-solid cells only (without a mask every cell counts). A lattice that takes the
+ * split step (xac_lattice_tune) on its own holds 32 bytes more per non-solid cell. */
 int xac_batch_open(int precision, xac_batch **out);
 int xac_batch_admit(xac_batch *batch, const xac_desc *design, int *slot, void *stream);
 int xac_batch_advance(xac_batch *batch, const xac_run_opts *opts, long long steps, int *n_finished, int *slots,

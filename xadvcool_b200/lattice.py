@@ -108,8 +108,8 @@ class Lattice:
         _capi.call("xac_lattice_tune", self._h, int(block), int(variant))
 
     def pattern_copy_us(self, launches: int = 200) -> float:
-        """Microseconds per launch of a kernel that moves exactly the step's populations with no arithmetic (the
-        memory-pattern floor of the step for this design); leaves the lattice at the cold start (step 0)."""
+        """Microseconds per launch of a kernel that moves exactly the step's populations in the one-pass step's access
+        pattern with no arithmetic; leaves the lattice at the cold start (step 0)."""
         us = C.c_double()
         with torch.cuda.device(self.device):
             _capi.call("xac_lattice_pattern_copy", self._h, int(launches), C.byref(us), stream_ptr(self.device))

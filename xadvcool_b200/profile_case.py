@@ -14,8 +14,8 @@ after few prior launches.
 
     python -m xadvcool_b200.profile_case --conv b3b --steps 2   # one surrogate convolution layer, batch 4
 
-runs the named layer of the warm-start surrogate (forward convolution on the tensor-core kernel, the 148x128x32
-volume padded to 152 in x) inside the profiler range, after one untimed launch.
+runs the named layer of the warm-start surrogate (forward convolution on the tensor-core kernel, or its weight gradient
+with --grad; the 148x128x32 volume padded to 152 in x) inside the profiler range, after one untimed launch.
 """
 from __future__ import annotations
 
@@ -33,21 +33,23 @@ CONV_LAYERS = {  # name: (D, H, W, Ci, Co) at batch 4
 }
 
 
-def conv_case(name, steps):
+def conv_case(name, steps, grad):
     from . import surrogate as S
     D, H, W, Ci, Co = CONV_LAYERS[name]
     g = torch.Generator(device="cuda").manual_seed(0)
     x = torch.randn((4, D, H, W, Ci), device="cuda", generator=g).to(S.BF16)
     w = (torch.randn((27, Co, Ci), device="cuda", generator=g) * 0.05).to(S.BF16)
     b = torch.zeros(Co, device="cuda")
-    S.conv_forward(x, w, b, 3)
+    y = S.conv_forward(x, w, b, 3)
+    call = (lambda: S.conv_weight_grad(x, y, 3, True)[0]) if grad else (lambda: S.conv_forward(x, w, b, 3))
+    call()
     torch.cuda.synchronize()
     torch.cuda.profiler.start()
     for _ in range(steps):
-        y = S.conv_forward(x, w, b, 3)
+        out = call()
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
-    print(f"conv case {name}: {tuple(y.shape)}, status {S.kernel_status()}")
+    print(f"conv case {name}: {tuple(out.shape)}, status {S.kernel_status()}")
 
 
 def main(argv=None):
@@ -61,9 +63,10 @@ def main(argv=None):
     ap.add_argument("--block", type=int, default=128)
     ap.add_argument("--variant", type=int, default=0)
     ap.add_argument("--conv", choices=sorted(CONV_LAYERS), help="profile one surrogate convolution layer instead")
+    ap.add_argument("--grad", action="store_true", help="the layer's weight gradient instead of its forward convolution")
     a = ap.parse_args(argv)
     if a.conv:
-        conv_case(a.conv, a.steps)
+        conv_case(a.conv, a.steps, a.grad)
         return
     mask, hs, u_in, _ = designs.gyroid_design(0)
     lat = Lattice(mask, heat_source=hs, tau_fluid=0.55, u_inlet_val=u_in, precision=a.precision)
